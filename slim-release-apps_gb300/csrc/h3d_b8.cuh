@@ -1,4 +1,5 @@
-// Batched BLOCK8 Kaczmarz double sweep over a table of problems (h3d_b8batch.cu).
+// Batched BLOCK8 Kaczmarz double sweep over a table of problems (h3d_b8batch.cu; the complex64
+// kernel in h3d_b8slab.cu).
 //
 // One launch per block parity covers every (problem, block, group of R right-hand sides) of
 // the batch: problems may differ in grid size, PML, wavenumber (frequency) and mode, and each
@@ -21,8 +22,9 @@ namespace h3d {
 template <typename T>
 struct B8Prob {
     Op<T> op;
-    const cplx<T> *coef;  // 12^3-block stored coefficients (store_block8_coefs layout)
-    const T *rinv8;       // 1/||a_i||^2 in the same block- and colour-major order, 64 per slab
+    const cplx<T> *coef;  // complex128: 12^3-block stored coefficients (store_block8_coefs layout)
+    const T *rinv8;       // complex128: 1/||a_i||^2 in the same block- and colour-major order, 64 per slab
+    const T *rec;         // complex64: block records (h3d_b8slab.cuh)
     long long col0;       // element offset of the problem's first column in x and b
     long long cstride;    // elements between two of its columns (its N)
     int c0;               // batch index of its first column (active flags)
@@ -36,8 +38,8 @@ struct B8Prob {
 // Compiled (precision, R, S) configurations of the batched kernel.
 struct B8Cfg {
     int r;    // right-hand sides per CTA
-    int rpt;  // right-hand sides per thread (64 r / rpt threads)
-    int s;    // depth of the coefficient ring
+    int rpt;  // right-hand sides per thread (complex128: 64 r / rpt threads)
+    int s;    // depth of the coefficient ring (complex64: none)
 };
 int b8_num_cfgs(bool fp64);
 B8Cfg b8_cfg(bool fp64, int c);
@@ -53,6 +55,7 @@ struct B8Batch {
     std::vector<Item> items;
     std::vector<std::unique_ptr<DevBuf>> coefs, rinvs;
     DevBuf desc, starts, errb;
+    B8Prob<T> first;                          // host copy of the first problem's descriptor
     int cfg = -1;
     long long nctas[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     int *err = nullptr;                       // device status: H3D_ERR_TIMEOUT after an expired wait
@@ -60,6 +63,13 @@ struct B8Batch {
     int verbose = 0;
 
     void add(const Op<T> &op, bool adj, long long col0, int c0, int nrhs) { items.push_back({op, adj, col0, c0, nrhs}); }
+    // Any problem with a complex wavenumber.
+    bool any_wnc() const
+    {
+        for (const Item &it : items)
+            if (it.op.wni) return true;
+        return false;
+    }
     // Device bytes setup() allocates: stored coefficients and block-ordered row norms.
     size_t bytes_needed() const;
     // Store every problem's coefficients and inverse row norms; clear the status word.

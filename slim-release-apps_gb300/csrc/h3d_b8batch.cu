@@ -2,6 +2,9 @@
 // of any sizes, the stored coefficients of each colour staged by bulk copies into a ring of
 // shared-memory buffers that complete on mbarriers.
 //
+// This file: the work list, the tuner, and the complex128 kernel on stored coefficients; the
+// complex64 kernel, which forms its coefficients, is in h3d_b8slab.cu.
+//
 // Row order and arithmetic are those of the BLOCK8 sweep (h3d_block8.cu, h3d_blockrow.cuh):
 // 12^3 blocks in eight parity classes, 27 colours inside a block, forward then backward
 // (Helm3dkaczswp_mex.c:60-120 with another row order).  What changes is how work and data
@@ -11,8 +14,8 @@
 //    (groups of R right-hand sides) CTAs, problem-major, block-major, group fastest (the CTAs
 //    of one block sit side by side and share its coefficient slabs through L2).  A CTA finds
 //    its problem by a binary search over the per-parity prefix counts.
-//  * Staging.  Thread 0 issues, per colour step, one cp.async.bulk of the colour's 13.8 KB
-//    coefficient slab (complex64; 27.6 KB complex128) and one of its 64 inverse row norms,
+//  * Staging.  Thread 0 issues, per colour step, one cp.async.bulk of the colour's 27.6 KB
+//    coefficient slab and one of its 64 inverse row norms,
 //    both completing on the step's mbarrier, S steps ahead into an S-deep ring; no other
 //    thread spends instructions on the copies.  Interior blocks (all PML values 1, real
 //    wavenumber) form their real coefficients from the staged wavenumber box instead and
@@ -29,6 +32,7 @@
 #include <tuple>
 
 #include "h3d_b8.cuh"
+#include "h3d_b8slab.cuh"
 #include "h3d_blockrow.cuh"
 #include "h3d_kernels.cuh"
 
@@ -344,9 +348,9 @@ __global__ void rinv8_kernel(const T *__restrict__ rinv, T *__restrict__ rinv8, 
 }
 
 // Compiled configurations (R right-hand sides per CTA, RPT per thread, ring depth S):
-// complex64 with a 3-deep ring; complex128 with a 2-deep ring (its R = 4 boxes would exceed a
-// CTA's 227 KB of shared memory).
-const B8Cfg kCfgF32[] = {{1, 1, 3}, {2, 1, 3}, {4, 1, 3}, {4, 2, 3}, {8, 1, 3}, {8, 2, 3}};
+// complex64 on the slab kernel (no ring); complex128 with a 2-deep ring (its R = 4 boxes would
+// exceed a CTA's 227 KB of shared memory).
+const B8Cfg kCfgF32[] = {{1, 1, 0}, {2, 2, 0}};
 const B8Cfg kCfgF64[] = {{1, 1, 2}, {2, 1, 2}, {2, 2, 2}};
 
 template <typename T, int R, int RPT, int S>
@@ -368,30 +372,23 @@ int launch_b8(const B8Prob<T> *probs, const int *starts, int nprob, long long nc
 }
 
 template <typename T>
-int launch_b8_cfg(int cfg, const B8Prob<T> *probs, const int *starts, int nprob, long long nctas, cplx<T> *x,
-                  const cplx<T> *b, T w, const int *active, int par, int backward, int nsteps, int *err,
+int launch_b8_cfg(int cfg, bool wnc, const B8Prob<T> &one, const B8Prob<T> *probs, const int *starts, int nprob, long long nctas, cplx<T> *x,
+                  const cplx<T> *b, T w, const int *active, int par, int pass, bool chained, int *err,
                   unsigned long long limit_ns, int selftest, cudaStream_t st)
 {
-#define H3D_B8_ARGS probs, starts, nprob, nctas, x, b, w, active, par, backward, nsteps, err, limit_ns, selftest, st
     if constexpr (sizeof(T) == 4) {
-        switch (cfg) {
-        case 0: return launch_b8<T, 1, 1, 3>(H3D_B8_ARGS);
-        case 1: return launch_b8<T, 2, 1, 3>(H3D_B8_ARGS);
-        case 2: return launch_b8<T, 4, 1, 3>(H3D_B8_ARGS);
-        case 3: return launch_b8<T, 4, 2, 3>(H3D_B8_ARGS);
-        case 4: return launch_b8<T, 8, 1, 3>(H3D_B8_ARGS);
-        case 5: return launch_b8<T, 8, 2, 3>(H3D_B8_ARGS);
-        default: break;
-        }
+        return launch_slab(kCfgF32[cfg].r, wnc, one, probs, starts, nprob, nctas, x, b, w, active, par, pass,
+                           chained, st);
     } else {
+#define H3D_B8_ARGS probs, starts, nprob, nctas, x, b, w, active, par, pass == 1, pass == 2 ? 54 : 27, err, limit_ns, selftest, st
         switch (cfg) {
         case 0: return launch_b8<T, 1, 1, 2>(H3D_B8_ARGS);
         case 1: return launch_b8<T, 2, 1, 2>(H3D_B8_ARGS);
         case 2: return launch_b8<T, 2, 2, 2>(H3D_B8_ARGS);
         default: break;
         }
-    }
 #undef H3D_B8_ARGS
+    }
     set_error("batched BLOCK8 configuration %d out of range", cfg);
     return H3D_ERR_BAD_ARG;
 }
@@ -421,7 +418,8 @@ size_t B8Batch<T>::bytes_needed() const
         int NI, NJ, NK;
         block_counts(it.op, &NI, &NJ, &NK);
         const size_t nslab = (size_t)NI * NJ * NK * 27;
-        tot += nslab * 27 * kNR * sizeof(cplx<T>) + nslab * kNR * sizeof(T) + (size_t)it.op.N * sizeof(T);
+        if (sizeof(T) == 8) tot += nslab * 27 * kNR * sizeof(cplx<T>) + nslab * kNR * sizeof(T) + (size_t)it.op.N * sizeof(T);
+        else tot += slab_record_bytes(NI, NJ, NK, any_wnc());
     }
     return tot;
 }
@@ -443,6 +441,13 @@ int B8Batch<T>::setup(cudaStream_t st)
         if (nslab * kNR > 0x7fffffffLL * 64LL) {
             set_error("grid too large for the batched BLOCK8 sweep");
             return H3D_ERR_NSIZE;
+        }
+        if constexpr (sizeof(T) == 4) {  // the slab kernel forms its coefficients: block records only
+            auto rb = std::make_unique<DevBuf>();
+            if ((rc = rb->alloc(slab_record_bytes(NI, NJ, NK, any_wnc()), st))) return rc;
+            if ((rc = launch_slab_pack(it.op, it.adj, NI, NJ, NK, any_wnc(), rb->as<T>(), st))) return rc;
+            rinvs.push_back(std::move(rb));
+            continue;
         }
         auto cb = std::make_unique<DevBuf>();
         auto rb = std::make_unique<DevBuf>();
@@ -483,8 +488,12 @@ int B8Batch<T>::configure(int c, cudaStream_t st)
         B8Prob<T> &d = h[i];
         std::memset(&d, 0, sizeof d);
         d.op = it.op;
-        d.coef = coefs[i]->as<cplx<T>>();
-        d.rinv8 = rinvs[i]->as<T>();
+        if (sizeof(T) == 8) {
+            d.coef = coefs[i]->as<cplx<T>>();
+            d.rinv8 = rinvs[i]->as<T>();
+        } else {
+            d.rec = rinvs[i]->as<T>();
+        }
         d.col0 = it.col0;
         d.cstride = it.op.N;
         d.c0 = it.c0;
@@ -515,6 +524,7 @@ int B8Batch<T>::configure(int c, cudaStream_t st)
     // pageable sources: staged before the calls return
     H3D_CUDA_TRY(cudaMemcpyAsync(desc.p, h.data(), sizeof(B8Prob<T>) * np, cudaMemcpyHostToDevice, st));
     H3D_CUDA_TRY(cudaMemcpyAsync(starts.p, hs.data(), sizeof(int) * hs.size(), cudaMemcpyHostToDevice, st));
+    first = h[0];
     cfg = c;
     return H3D_OK;
 }
@@ -535,13 +545,22 @@ int B8Batch<T>::dsweep(cplx<T> *x, const cplx<T> *b, T w, const int *active, cud
         return H3D_ERR_BAD_ARG;
     }
     const int np = (int)items.size();
+    const bool wnc = any_wnc();
+    // Overlapping a launch's prologue with the one before pays while both fit the device at one CTA
+    // per SM (61^3: 212 -> 189 us per double sweep); beyond that the early CTAs crowd the SMs that
+    // free up first (161 x 161 x 81, 147-196 CTAs a launch: 259 -> 311 us).
+    int dev = 0, sms = 0;
+    H3D_CUDA_TRY(cudaGetDevice(&dev));
+    H3D_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     // forward parities 0..6, parity 7 up and down in one launch, backward parities 6..0
+    long long before = -1;  // CTAs of the launch before, while this sweep has one
     for (int pp = 0; pp < 15; ++pp) {
         const int par = pp < 8 ? pp : 14 - pp;
         if (!nctas[par]) continue;
-        int rc = launch_b8_cfg<T>(cfg, desc.as<B8Prob<T>>(), starts.as<int>(), np, nctas[par], x, b, w, active, par,
-                                  pp < 8 ? 0 : 1, pp == 7 ? 54 : 27, err, wait_limit_ns, selftest, st);
+        int rc = launch_b8_cfg<T>(cfg, wnc, first, desc.as<B8Prob<T>>(), starts.as<int>(), np, nctas[par], x, b, w, active,
+                                  par, pp < 7 ? 0 : pp == 7 ? 2 : 1, before >= 0 && before + nctas[par] <= sms, err, wait_limit_ns, selftest, st);
         if (rc) return rc;
+        before = nctas[par];
     }
     H3D_CUDA_TRY(cudaGetLastError());
     return H3D_OK;

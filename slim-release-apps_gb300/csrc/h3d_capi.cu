@@ -36,8 +36,8 @@ static int kacz_sweep_t(const Op<T> &op, cplx<T> *x, const cplx<T> *b, int nrhs,
     }
     const bool blk12 = !block || block[0] == 0 || (block[0] == 12 && block[1] == 12 && block[2] == 12);
     if (order == H3D_ORDER_BLOCK8 && blk12) {
-        // the batched BLOCK8 kernel on one problem (stored coefficients, bulk-copied slabs);
-        // its status word is read back, so this call synchronises the stream
+        // the batched BLOCK8 kernel on one problem; complex128 (stored coefficients, bulk-copied
+        // slabs) reads its status word back, so that call synchronises the stream
         B8Batch<T> batch;
         batch.add(op, adj, 0, 0, nrhs);
         int rc = batch.setup(st);
@@ -55,6 +55,7 @@ static int kacz_sweep_t(const Op<T> &op, cplx<T> *x, const cplx<T> *b, int nrhs,
                 if (k >= 0 && k < b8_num_cfgs(fp64)) c = k;
             }
             if ((rc = batch.configure(c, st)) || (rc = batch.dsweep(x, b, w, nullptr, st))) return rc;
+            if (!fp64) return H3D_OK;  // the complex64 kernel has no waits
             int status = 0;
             H3D_CUDA_TRY(cudaMemcpyAsync(&status, batch.err, sizeof(int), cudaMemcpyDeviceToHost, st));
             H3D_CUDA_TRY(cudaStreamSynchronize(st));
@@ -305,18 +306,18 @@ int h3d_check_wait_timeout(double limit_ms)
     int rc = [&]() -> int {
         DevBuf wn, x;
         int r;
-        if ((r = wn.alloc(sizeof(float) * (size_t)N, st)) || (r = x.alloc(sizeof(cplx<float>) * (size_t)N, st))) return r;
+        if ((r = wn.alloc(sizeof(double) * (size_t)N, st)) || (r = x.alloc(sizeof(cplx<double>) * (size_t)N, st))) return r;
         const double k2 = std::pow(2.0 * M_PI * 5.0 / 2000.0, 2);
-        std::vector<float> h((size_t)N, (float)k2);
-        H3D_CUDA_TRY(cudaMemcpyAsync(wn.p, h.data(), sizeof(float) * (size_t)N, cudaMemcpyHostToDevice, st));
-        H3D_CUDA_TRY(cudaMemsetAsync(x.p, 0, sizeof(cplx<float>) * (size_t)N, st));
-        Op<float> op;
-        if ((r = make_op_f32(&g, wn.as<float>(), nullptr, &op))) return r;
-        B8Batch<float> batch;
+        std::vector<double> h((size_t)N, k2);
+        H3D_CUDA_TRY(cudaMemcpyAsync(wn.p, h.data(), sizeof(double) * (size_t)N, cudaMemcpyHostToDevice, st));
+        H3D_CUDA_TRY(cudaMemsetAsync(x.p, 0, sizeof(cplx<double>) * (size_t)N, st));
+        Op<double> op;
+        if ((r = make_op_f64(&g, wn.as<double>(), nullptr, &op))) return r;
+        B8Batch<double> batch;
         batch.add(op, false, 0, 0, 1);
         if ((r = batch.setup(st)) || (r = batch.configure(0, st))) return r;
         batch.wait_limit_ns = (unsigned long long)(limit_ms * 1e6);
-        if ((r = batch.dsweep(x.as<cplx<float>>(), nullptr, 1.5f, nullptr, st, 1))) return r;
+        if ((r = batch.dsweep(x.as<cplx<double>>(), nullptr, 1.5, nullptr, st, 1))) return r;
         H3D_CUDA_TRY(cudaMemcpyAsync(&status, batch.err, sizeof(int), cudaMemcpyDeviceToHost, st));
         H3D_CUDA_TRY(cudaStreamSynchronize(st));
         return H3D_OK;

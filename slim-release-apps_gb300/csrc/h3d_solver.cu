@@ -565,7 +565,9 @@ static bool use_batched_block8(const std::vector<SolveProb> &P, const h3d_solve_
     const size_t cs = o.precision == H3D_PREC_FP64 ? 16 : 8;
     for (const SolveProb &p : P) {
         const size_t nb = (size_t)((p.g.n[0] + 11) / 12) * ((p.g.n[1] + 11) / 12) * ((p.g.n[2] + 11) / 12) * 27 * 64;
-        need += nb * (27 * cs + cs / 2) + (size_t)p.g.n[0] * p.g.n[1] * p.g.n[2] * (cs / 2);
+        // complex128: stored coefficients and row norms; complex64: block records (at most 7440 floats)
+        if (o.precision == H3D_PREC_FP64) need += nb * (27 * cs + cs / 2) + (size_t)p.g.n[0] * p.g.n[1] * p.g.n[2] * (cs / 2);
+        else need += nb / (27 * 64) * 7440 * sizeof(float);
     }
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
