@@ -10,7 +10,7 @@
 //    coefficient rule shared with every other kernel (row_coefs).
 //  * band_mvp_kernel: y = A x for any ndiags <= kMaxBands (Hmvp_MT_mex.c:53-73), couplings
 //    outside 0 <= i + offset < N skipped as the reference does; one thread per (row, rhs).
-//  * band_lex_kernel: the Kaczmarz double sweep of sweep_MT_mex.c:55-97 (rows 0..N-1, then
+//  * the sweep (h3d_lex.cu): the Kaczmarz double sweep of sweep_MT_mex.c:55-97 (rows 0..N-1, then
 //    N-1..0).  The rows run as the hyperplanes t = i + 3j + 9k of the grid, the schedule of
 //    the matrix-free LEX sweep: rows of one hyperplane share no grid neighbour, and every
 //    earlier row that shares one has a smaller t, so the result is the sequential one as
@@ -71,52 +71,6 @@ __global__ void __launch_bounds__(256) band_mvp_kernel(const cplx<T> *__restrict
         if (q >= 0 && q < N) cmac(acc, a[k], xs[q]);
     }
     y[s * N + row] = acc;
-}
-
-// One hyperplane t = i + 3j + 9k of the band sweep; (i, j, k) from (t, j) as in the LEX
-// kernel.  rn: squared row norms (NULL: the sum over all 27 bands, opBandStorage.m:139-144).
-template <typename T>
-__global__ void __launch_bounds__(128) band_lex_kernel(int nx, int ny, int nz, long long N,
-                                                       const cplx<T> *__restrict__ coef, BandOffsets offs,
-                                                       const T *__restrict__ rn, cplx<T> *x,
-                                                       const cplx<T> *__restrict__ b, int nrhs, int t, T w)
-{
-    const int kk = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (j >= ny) return;
-    const int r = t - 3 * j;  // = i + 9k
-    if (r < 0) return;
-    const int kmax = min(r / 9, nz - 1);
-    const int kmin = r - (nx - 1) <= 0 ? 0 : (r - (nx - 1) + 8) / 9;
-    const int k = kmin + kk;
-    if (k > kmax) return;
-    const int i = r - 9 * k;
-    const long long row = i + (long long)nx * (j + (long long)ny * k);
-    const uint32_t m = inside_mask(i, j, k, nx, ny, nz);
-    cplx<T> c[27];
-    const cplx<T> *a = coef + 27 * row;
-#pragma unroll
-    for (int q = 0; q < 27; ++q) c[q] = a[q];
-    T nrm;
-    if (rn) {
-        nrm = rn[row];
-    } else {
-        nrm = T(0);
-#pragma unroll
-        for (int q = 0; q < 27; ++q) nrm += cabs2(c[q]);
-    }
-    for (int s = 0; s < nrhs; ++s) {
-        cplx<T> *xs = x + (long long)s * N;
-        cplx<T> atx = mk<T>(T(0), T(0));
-#pragma unroll
-        for (int q = 0; q < 27; ++q)
-            if ((m >> offs.t[q]) & 1u) cmac(atx, c[q], xs[row + offs.v[q]]);
-        const cplx<T> bv = b ? b[(long long)s * N + row] : mk<T>(T(0), T(0));
-        const cplx<T> d = mk<T>(w * (bv.re - atx.re) / nrm, w * (bv.im - atx.im) / nrm);
-#pragma unroll
-        for (int q = 0; q < 27; ++q)
-            if ((m >> offs.t[q]) & 1u) cmac_cb(xs[row + offs.v[q]], d, c[q]);
-    }
 }
 
 // The 27 linear offsets of grid g in band order t = (dx+1) + 3(dy+1) + 9(dz+1).
@@ -245,36 +199,21 @@ extern "C" int h3d_band_sweep(const h3d_grid *g, const void *coef, const int64_t
         offs.v[k] = offsets[k];
         offs.t[k] = (unsigned char)dir;
     }
-    const int nx = g->n[0], ny = g->n[1], nz = g->n[2];
-    const long long N = (long long)nx * ny * nz;
-    const int tmax = (nx - 1) + 3 * (ny - 1) + 9 * (nz - 1);
-    const int kw = (nx + 8) / 9 + 1;  // k values per (t, j)
-    const dim3 blk(32, 4);
-    const dim3 grd((kw + 31) / 32, (ny + 3) / 4);
-    if (grd.y > 65535) {
+    if ((g->n[1] + 3) / 4 > 65535) {
         set_error("h3d_band_sweep: ny too large");
         return H3D_ERR_NSIZE;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int tt = 0; tt <= tmax; ++tt) {
-            const int t = pass == 0 ? tt : tmax - tt;
-            if (dtype == H3D_C128)
-                band_lex_kernel<double><<<grd, blk, 0, st>>>(nx, ny, nz, N, (const cplx<double> *)coef, offs,
-                                                             (const double *)row_norms, (cplx<double> *)x,
-                                                             (const cplx<double> *)b, nrhs, t, w);
-            else if (dtype == H3D_C64)
-                band_lex_kernel<float><<<grd, blk, 0, st>>>(nx, ny, nz, N, (const cplx<float> *)coef, offs,
-                                                            (const float *)row_norms, (cplx<float> *)x,
-                                                            (const cplx<float> *)b, nrhs, t, (float)w);
-            else {
-                set_error("h3d_band_sweep: unknown dtype %d", dtype);
-                return H3D_ERR_BAD_ARG;
-            }
-        }
-    }
-    H3D_CUDA_TRY(cudaGetLastError());
-    return H3D_OK;
+    if (dtype == H3D_C128)
+        return sweep_lex_stored<double>(g->n[0], g->n[1], g->n[2], (const cplx<double> *)coef, offs.t,
+                                        (const double *)row_norms, false, (cplx<double> *)x, (const cplx<double> *)b,
+                                        nrhs, w, nullptr, st);
+    if (dtype == H3D_C64)
+        return sweep_lex_stored<float>(g->n[0], g->n[1], g->n[2], (const cplx<float> *)coef, offs.t,
+                                       (const float *)row_norms, false, (cplx<float> *)x, (const cplx<float> *)b, nrhs,
+                                       (float)w, nullptr, st);
+    set_error("h3d_band_sweep: unknown dtype %d", dtype);
+    return H3D_ERR_BAD_ARG;
 }
 
 // ---------------------------------------------------------------------------------------

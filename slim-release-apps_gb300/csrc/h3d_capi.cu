@@ -34,6 +34,18 @@ static int kacz_sweep_t(const Op<T> &op, cplx<T> *x, const cplx<T> *b, int nrhs,
         }
         (void)cudaGetLastError();  // out of memory is not sticky: fall back to the tile kernel
     }
+    // LEX on stored coefficients where they fit: a plane of rows then takes a warp's short chain per
+    // row instead of a thread's 600 FP64 instructions.  Otherwise the kernel that forms them per row.
+    if (order == H3D_ORDER_LEX) {
+        DevBuf cb, rb;
+        if (cb.alloc(sizeof(cplx<T>) * 27 * (size_t)op.N, st) == H3D_OK &&
+            rb.alloc(sizeof(T) * (size_t)op.N, st) == H3D_OK) {
+            int rc = store_lex_coefs<T>(op, adj, cb.as<cplx<T>>(), rb.as<T>(), st);
+            if (!rc) rc = launch_sweep<T>(op, x, b, nrhs, w, adj, order, block, nullptr, st, rb.as<T>(), -1, cb.as<cplx<T>>());
+            return rc;
+        }
+        (void)cudaGetLastError();
+    }
     const bool blk12 = !block || block[0] == 0 || (block[0] == 12 && block[1] == 12 && block[2] == 12);
     if (order == H3D_ORDER_BLOCK8 && blk12) {
         // the batched BLOCK8 kernel on one problem; complex128 (stored coefficients, bulk-copied

@@ -43,6 +43,16 @@ int launch_sweep(const Op<T> &op, cplx<T> *x, const cplx<T> *b, int nrhs, T w, b
                  int order, const int32_t *block, const int *active, cudaStream_t st,
                  const T *rinv = nullptr, int shape = -1, const cplx<T> *coef = nullptr);
 
+// h3d_lex.cu: the lexicographic sweep on stored coefficients ([row][27], 27 N complex values).
+// store_lex_coefs: t = (dx+1) + 3(dy+1) + 9(dz+1) and 1/||a_i||^2.  sweep_lex_stored: dirs gives the
+// direction t of each coefficient column (null: in order); scale holds 1/||a_i||^2 (inverse) or
+// ||a_i||^2 (null: formed from the row); couplings that leave the grid are skipped.
+template <typename T>
+int store_lex_coefs(const Op<T> &op, bool adj, cplx<T> *coef, T *rinv, cudaStream_t st);
+template <typename T>
+int sweep_lex_stored(int nx, int ny, int nz, const cplx<T> *coef, const unsigned char dirs[27], const T *scale,
+                     bool inverse, cplx<T> *x, const cplx<T> *b, int nrhs, T w, const int *active, cudaStream_t st);
+
 // h3d_sweep_direct.cu: COLOUR27 on stored row coefficients (27 N complex values, colour-major).
 template <typename T>
 int store_row_coefs(const Op<T> &op, bool adj, cplx<T> *coef, cudaStream_t st);

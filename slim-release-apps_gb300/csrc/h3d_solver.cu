@@ -188,7 +188,18 @@ struct CgRun {
         if ((rc = parts.alloc(sizeof(double) * 2 * (size_t)s.G * nrhs, st))) return rc;
         s.part = parts.as<double>();
         if (b8) return H3D_OK;  // the batch holds its own coefficients and row norms
-        if (order != H3D_ORDER_LEX) {
+        if (order == H3D_ORDER_LEX) {  // stored coefficients when they take at most half of the free memory
+            size_t fr = 0, tot = 0;
+            const size_t bytes = sizeof(cplx<T>) * 27 * (size_t)N;
+            if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && bytes <= fr / 2 && coefs.alloc(bytes, st) == H3D_OK &&
+                norms.alloc(sizeof(T) * (size_t)N, st) == H3D_OK) {
+                coef = coefs.as<cplx<T>>();
+                rinv = norms.as<T>();
+                if ((rc = store_lex_coefs<T>(op, adj, coef, rinv, st))) return rc;
+                launches += 1;
+            }
+            (void)cudaGetLastError();
+        } else {
             if ((rc = norms.alloc(sizeof(T) * (size_t)N, st))) return rc;
             rinv = norms.as<T>();
             if ((rc = row_inv_norms<T>(op, adj, rinv, st))) return rc;
@@ -371,7 +382,7 @@ struct CgRun {
     // Stored coefficients for the sweep launches (null: the chosen kernel does not use them).
     const cplx<T> *cf() const
     {
-        if (order == H3D_ORDER_BLOCK8) return coef;
+        if (order == H3D_ORDER_BLOCK8 || order == H3D_ORDER_LEX) return coef;
         return (order == H3D_ORDER_COLOUR27 && shape == num_tile_shapes()) ? coef : nullptr;
     }
 

@@ -1,5 +1,6 @@
 // Kaczmarz double sweeps of the 27-point Helmholtz operator: row-order dispatch and the
-// exact-LEX hyperplane kernel (the COLOUR27 and BLOCK kernels live in their own files).
+// exact-LEX hyperplane kernel that forms its coefficients (the LEX sweep on stored coefficients, the
+// COLOUR27 and the BLOCK kernels live in their own files).
 //
 // Reference semantics: do_Hmvp (tools/algorithms/3DFreqModeling/Helm3d_27pt.h:827-875) and
 // do_sweep (Helm3dkaczswp_mex.c:60-120).  Layout: interleaved complex, x fastest,
@@ -57,7 +58,9 @@ static int sweep_dispatch(const Op<T> &op, cplx<T> *x, const cplx<T> *b, int nrh
                           const T *rinv, int shape, const cplx<T> *coef)
 {
     int rc = H3D_OK;
-    if (order == H3D_ORDER_LEX) {
+    if (order == H3D_ORDER_LEX && coef && rinv) {
+        rc = sweep_lex_stored<T>(op.nx, op.ny, op.nz, coef, nullptr, rinv, true, x, b, nrhs, w, active, st);
+    } else if (order == H3D_ORDER_LEX) {
         rc = sweep_lex_pass<T, ADJ, WNC>(op, x, b, nrhs, w, active, false, st);
         if (!rc) rc = sweep_lex_pass<T, ADJ, WNC>(op, x, b, nrhs, w, active, true, st);
     } else if (order == H3D_ORDER_COLOUR27 && coef && rinv) {
