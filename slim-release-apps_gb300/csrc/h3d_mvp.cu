@@ -17,6 +17,7 @@
 // ||r||^2 and ||b||^2 (RESID).
 #include "h3d_internal.cuh"
 #include "h3d_kernels.cuh"
+#include "h3d_mvpflat.cuh"
 #include "h3d_reduce.cuh"
 #include "h3d_planes.cuh"
 
@@ -266,6 +267,83 @@ static dim3 zmarch_grid(const Op<T> &op, int nrhs, int *kz, int *nchunks)
     return dim3((unsigned)gx, (unsigned)gy, *nchunks * nrhs);
 }
 
+// The flat kernel's z split: an SM works off its CTAs at a fixed rate whatever runs side by side,
+// but the last one alone keeps the FP64 unit only 70% busy; a CTA's time grows with the planes it
+// marches (its own, and about half the work for either halo plane): the split minimises
+// (CTAs of the fullest SM + 0.4) x (chunk + 1).
+static int device_sms()
+{
+    static int cache[64] = {0};
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        cudaGetLastError();
+        return 1;
+    }
+    if (cache[dev] == 0) {
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) {
+            cudaGetLastError();
+            v = 1;
+        }
+        cache[dev] = v;
+    }
+    return cache[dev];
+}
+
+// RESID: at most the partial sums per right-hand side of the tiled kernel's grid, so that what fits a
+// fixed partial-sum buffer with that kernel fits it with this one.
+template <typename T, bool RESID>
+static dim3 flat_grid(const Op<T> &op, int nrhs, int *kz, int *nchunks)
+{
+    const long long gx = ((long long)op.nx * op.ny + kFT - 1) / kFT, sms = device_sms();
+    long long most = 65535LL * gx;
+    if (RESID) {
+        const dim3 g = zmarch_grid<T, RESID>(op, nrhs, kz, nchunks);
+        most = (long long)g.x * g.y * *nchunks;
+    }
+    int best_kz = op.nz;
+    long long best = -1;
+    const int nmax = op.nz < 64 ? op.nz : 64;
+    for (int n = 1; n <= nmax; ++n) {
+        const int k = (op.nz + n - 1) / n;
+        const long long nch = (op.nz + k - 1) / k, ctas = gx * nch * nrhs;
+        if (nch > 1 && (nch * nrhs > 65535 || nch * gx > most)) break;
+        const long long cost = (5 * ((ctas + sms - 1) / sms) + 2) * (k + 1);
+        if (best < 0 || cost < best) {
+            best = cost;
+            best_kz = k;
+        }
+    }
+    *kz = best_kz;
+    *nchunks = (op.nz + best_kz - 1) / best_kz;
+    return dim3((unsigned)gx, (unsigned)(*nchunks * nrhs));
+}
+
+// Whether the flat kernel takes a grid: complex128 (bound by the FP64 unit), and staged planes (one
+// row more on either side of 256 points) that leave room for two CTAs per SM.  In complex64 the
+// column tiles are faster (201 x 201 x 101: 53 us against 89): what counts there is instructions, and
+// a row more on either side of 256 points is three times the copies of a 34 x 10 tile.
+template <typename T>
+static bool use_flat(const Op<T> &op)
+{
+    return sizeof(T) == 8 && flat_smem<double, false, true>(op.nx) <= 96 * 1024;
+}
+
+template <typename T, bool ADJ, bool DERIV, bool WNC, bool RESID>
+static int flat_launch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const cplx<T> *b, dim3 grd, int kz, int nch,
+                       double *part, cudaStream_t st)
+{
+    if constexpr (sizeof(T) == 8) {
+        const size_t smem = flat_smem<T, ADJ, WNC>(op.nx);
+        auto *kern = mvp_flat_kernel<T, ADJ, DERIV, WNC, RESID>;
+        if (smem > 48 * 1024)
+            H3D_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        auto aligned = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
+        const int vec = aligned(x) && aligned(op.wn) && (!WNC || aligned(op.wni));
+        kern<<<grd, kFT, smem, st>>>(op, x, y, b, kz, nch, vec, part);
+    }
+    return H3D_OK;
+}
+
 template <typename T, bool RESID>
 static int zmarch_dispatch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const cplx<T> *b, int nrhs,
                            bool adj, bool deriv, double *part, int parts, cudaStream_t st)
@@ -275,29 +353,37 @@ static int zmarch_dispatch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const 
         return H3D_ERR_NSIZE;
     }
     int kz, nch;
-    const dim3 grd = zmarch_grid<T, RESID>(op, nrhs, &kz, &nch);
+    const bool flat = use_flat(op);
+    const dim3 grd = flat ? flat_grid<T, RESID>(op, nrhs, &kz, &nch) : zmarch_grid<T, RESID>(op, nrhs, &kz, &nch);
     if ((long long)nch * nrhs > 65535) {
         set_error("too many right-hand sides for one launch");
         return H3D_ERR_BAD_ARG;
     }
-    if (RESID && (long long)grd.x * grd.y * nch != parts) {
+    const long long have = flat ? (long long)grd.x * nch : (long long)grd.x * grd.y * nch;
+    if (RESID && have != parts) {
         // the partial-sum buffer was sized for another grid: refuse rather than overrun it
         set_error("residual: %lld column blocks per right-hand side, buffer sized for %d",
-                  (long long)grd.x * grd.y * nch, parts);
+                  have, parts);
         return H3D_ERR_BAD_ARG;
     }
     const dim3 blk(kMX, kMY);
     const bool wnc = op.wni != nullptr;
-#define H3D_ZM(A, D, W) mvp_zmarch_kernel<T, A, D, W, RESID><<<grd, blk, 0, st>>>(op, x, y, b, kz, nch, part)
-    if (!adj && !deriv && !wnc) H3D_ZM(false, false, false);
-    else if (!adj && !deriv && wnc) H3D_ZM(false, false, true);
-    else if (!adj && deriv && !wnc) H3D_ZM(false, true, false);
-    else if (!adj && deriv && wnc) H3D_ZM(false, true, true);
-    else if (adj && !deriv && !wnc) H3D_ZM(true, false, false);
-    else if (adj && !deriv && wnc) H3D_ZM(true, false, true);
-    else if (adj && deriv && !wnc) H3D_ZM(true, true, false);
-    else H3D_ZM(true, true, true);
+    int rc = H3D_OK;
+#define H3D_ZM(A, D, W)                                                                        \
+    if (flat) rc = flat_launch<T, A, D, W, RESID>(op, x, y, b, grd, kz, nch, part, st);          \
+    else mvp_zmarch_kernel<T, A, D, W, RESID><<<grd, blk, 0, st>>>(op, x, y, b, kz, nch, part)
+    switch ((adj ? 4 : 0) + (deriv ? 2 : 0) + (wnc ? 1 : 0)) {
+    case 0: H3D_ZM(false, false, false); break;
+    case 1: H3D_ZM(false, false, true); break;
+    case 2: H3D_ZM(false, true, false); break;
+    case 3: H3D_ZM(false, true, true); break;
+    case 4: H3D_ZM(true, false, false); break;
+    case 5: H3D_ZM(true, false, true); break;
+    case 6: H3D_ZM(true, true, false); break;
+    default: H3D_ZM(true, true, true); break;
+    }
 #undef H3D_ZM
+    if (rc) return rc;
     H3D_CUDA_TRY(cudaGetLastError());
     return H3D_OK;
 }
@@ -312,6 +398,10 @@ int launch_mvp(const Op<T> &op, const cplx<T> *x, cplx<T> *y, int nrhs, bool adj
 int mvp_residual_parts(const Op<double> &op, int nrhs)
 {
     int kz, nch;
+    if (use_flat(op)) {
+        const dim3 g = flat_grid<double, true>(op, nrhs, &kz, &nch);
+        return (int)(g.x * nch);
+    }
     const dim3 g = zmarch_grid<double, true>(op, nrhs, &kz, &nch);
     return (int)(g.x * g.y * nch);
 }
