@@ -198,18 +198,23 @@ def check(status: int, where: str):
 def make_grid(n, h, npml) -> Grid:
     """``npml``: scalar, 3 values (same on both sides), 6 values (lo_x, hi_x, lo_y, hi_y,
     lo_z, hi_z) or the reference's 2x3 matrix (rows lo/hi, columns x/y/z)."""
-    import numpy as np
+    if type(npml) is int:            # the plain forms without numpy: this runs on every call
+        p = (npml,) * 6
+    elif type(npml) is tuple and len(npml) == 6 and all(type(q) is int for q in npml):
+        p = npml
+    else:
+        import numpy as np
 
-    p = np.asarray(npml)
-    if p.shape == (2, 3):
-        p = p.T.reshape(-1)          # column-major 2x3 -> lo_x, hi_x, lo_y, hi_y, lo_z, hi_z
-    p = p.astype(np.int64).ravel()
-    if p.size == 1:
-        p = np.repeat(p, 6)
-    elif p.size == 3:
-        p = np.repeat(p, 2)
-    if p.size != 6:
-        raise ValueError("npml must have 1, 3 or 6 entries or be 2x3")
+        p = np.asarray(npml)
+        if p.shape == (2, 3):
+            p = p.T.reshape(-1)          # column-major 2x3 -> lo_x, hi_x, lo_y, hi_y, lo_z, hi_z
+        p = p.astype(np.int64).ravel()
+        if p.size == 1:
+            p = np.repeat(p, 6)
+        elif p.size == 3:
+            p = np.repeat(p, 2)
+        if p.size != 6:
+            raise ValueError("npml must have 1, 3 or 6 entries or be 2x3")
     g = Grid()
     for a in range(3):
         g.n[a] = int(n[a])

@@ -14,6 +14,7 @@ else its adjoint; a complex ``wn`` selects the complex-wavenumber kernels.
 from __future__ import annotations
 
 import ctypes as C
+import math
 
 import torch
 
@@ -60,7 +61,7 @@ def _rhs(x: torch.Tensor, N: int):
     if x.shape[-1] != N:
         raise L.H3DError(L.ERR_XSIZE, "h3d", "x must have nx*ny*nz elements",
                          "SLIM_release_apps:tools:algorithms:ThreeDFreqModeling:Helm3dkaczswp_mex:Xsize")
-    P = 1 if x.dim() == 1 else int(torch.tensor(x.shape[:-1]).prod())
+    P = math.prod(x.shape[:-1])
     return x.contiguous(), P
 
 
