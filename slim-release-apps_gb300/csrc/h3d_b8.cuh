@@ -38,7 +38,7 @@ struct B8Prob {
 // Compiled (precision, R, S) configurations of the batched kernel.
 struct B8Cfg {
     int r;    // right-hand sides per CTA
-    int rpt;  // right-hand sides per thread (complex128: 64 r / rpt threads)
+    int rpt;  // right-hand sides per thread (complex128: 128 r / rpt threads)
     int s;    // depth of the coefficient ring (complex64: none)
 };
 int b8_num_cfgs(bool fp64);

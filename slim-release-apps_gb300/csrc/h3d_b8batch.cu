@@ -110,17 +110,21 @@ constexpr size_t b8_smem() { return 128 + (size_t)R * kNB * sizeof(cplx<T>) + ri
 // selftest != 0 (h3d_check_wait_timeout only): the first step's copies are announced on its
 // mbarrier but never issued, so that every wait of the first colour step expires.
 //
-// R right-hand sides per CTA; each thread projects one row of every colour for RPT of them,
-// from one load of the row's coefficients (64 R / RPT threads).
+// R right-hand sides per CTA; two lanes project one row of every colour for RPT of them, from one
+// load of the row's coefficients (128 R / RPT threads).  Two lanes, so that one right-hand side
+// runs four warps, one per SM sub-partition: each sub-partition has a quarter of the SM's FP64 unit (a
+// warp's FP64 instruction takes it 64 cycles), and with a lane per row the two warps of a
+// block left half of it idle (us per double sweep, one column, a lane per row -> two: 61^3 3450 ->
+// 2110, 161 x 161 x 81 3760 -> 2910).
 template <typename T, int R, int RPT, int S>
-__global__ void __launch_bounds__(kNR *R / RPT) sweep_b8_kernel(const B8Prob<T> *__restrict__ probs,
+__global__ void __launch_bounds__(2 * kNR *R / RPT) sweep_b8_kernel(const B8Prob<T> *__restrict__ probs,
                                                                 const int *__restrict__ starts, int nprob, cplx<T> *x,
                                                                 const cplx<T> *b, T w, const int *active, int par,
                                                                 int backward, int nsteps, int *err,
                                                                 unsigned long long limit_ns, int selftest)
 {
     static_assert(R % RPT == 0, "RPT must divide R");
-    constexpr int NT = kNR * R / RPT, SLAB = 27 * kNR;
+    constexpr int NT = 2 * kNR * R / RPT, SLAB = 27 * kNR;
     constexpr uint32_t SLABB = slab_bytes<T>(), RVB = rinv_bytes<T>();
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ B8Prob<T> sp;
@@ -192,7 +196,7 @@ __global__ void __launch_bounds__(kNR *R / RPT) sweep_b8_kernel(const B8Prob<T> 
 
     // the halo'd boxes of x (and the wavenumber box of an interior block), zero outside the grid,
     // one box row (14 points along x) at a time.  One right-hand side: a thread per row, its 14
-    // points unrolled (fewest instructions; the 64 threads have 196 rows to copy).  Several: a
+    // points unrolled (fewest instructions).  Several: a
     // half-warp per row, lane l on point l (the copies of a warp stay contiguous).
     const int i0 = bi0 - 1, j0 = bj0 - 1, k0 = bk0 - 1;
     constexpr int kRows = kPY * (kBS + 2);
@@ -234,10 +238,12 @@ __global__ void __launch_bounds__(kNR *R / RPT) sweep_b8_kernel(const B8Prob<T> 
     blk_cp_async_wait_all();
     __syncthreads();
 
-    // thread slot: row (u, v, w) of every colour, right-hand sides s0 + r0 .. s0 + r0 + RPT - 1
-    // (a half-warp spans (u, w): conflict-free box offsets, as the BLOCK8 kernel)
-    const int r0 = (tid / kNR) * RPT, row = tid % kNR;
-    const int u = row % 4, ww = (row / 4) % 4, v = row / 16;
+    // thread slot: half h of row (u, v, w) of every colour, right-hand sides s0 + r0 .. s0 + r0 + RPT - 1
+    // (a half-warp spans (u, w): conflict-free box offsets)
+    const int r0 = (tid / (2 * kNR)) * RPT, lane = tid & 31;
+    const int u = lane & 3, ww = (lane >> 2) & 3, v = (tid % (2 * kNR)) >> 5, row = u + 4 * ww + 16 * v;
+    const bool centre = lane < 16;
+    const int sg = centre ? 1 : -1;
     const unsigned mine = (act >> r0) & ((1u << RPT) - 1u);
     cplx<T> bv_n[RPT];
 #pragma unroll
@@ -261,30 +267,58 @@ __global__ void __launch_bounds__(kNR *R / RPT) sweep_b8_kernel(const B8Prob<T> 
         const bool ok = mbar_wait(smem_u32(bars + buf), (uint32_t)((qq / S) & 1), limit_ns);
         const int a = q % 3, bq = (q / 3) % 3, cq = q / 9;
         const int i = bi0 + a + 3 * u, j = bj0 + bq + 3 * v, k = bk0 + cq + 3 * ww;
-        if (ok && mine && i < op.nx && j < op.ny && k < op.nz) {
-            const T inv = rv[buf * kNR + row];
-            const int lc = (1 + a + 3 * u) + kPX * ((1 + bq + 3 * v) + kPY * (1 + cq + 3 * ww));
-            if (!interior) {
-                const cplx<T> *sc = reinterpret_cast<const cplx<T> *>(ring + (size_t)buf * SLABB);
-                cplx<T> c[27];
+        // the two halves of a row agree on `run`; every lane takes part in the exchange
+        const bool run = ok && mine && i < op.nx && j < op.ny && k < op.nz;
+        const int lc = (1 + a + 3 * u) + kPX * ((1 + bq + 3 * v) + kPY * (1 + cq + 3 * ww));
+        const T inv = run ? rv[buf * kNR + row] : T(0);
+        cplx<T> xv[RPT][14], part[RPT];
 #pragma unroll
-                for (int t = 0; t < 27; ++t) c[t] = sc[t * kNR + row];
-                // neighbours outside the grid keep reading zero: a row on a face of the grid
-                // scatters to its inside neighbours only
-                uint32_t m = 0x7ffffffu;
-                if (edge_block && (i == 0 || j == 0 || k == 0 || i == op.nx - 1 || j == op.ny - 1 || k == op.nz - 1))
-                    m = inside_mask(i, j, k, op.nx, op.ny, op.nz);
+        for (int kk = 0; kk < RPT; ++kk) part[kk] = mk<T>(T(0), T(0));
+        auto project = [&](int kk) {  // d of right-hand side kk from both halves' sums
+            cplx<T> t = part[kk];
+            t.re += __shfl_xor_sync(0xffffffffu, t.re, 16);
+            t.im += __shfl_xor_sync(0xffffffffu, t.im, 16);
+            return (w * inv) * (bv[kk] - t);
+        };
+        if (!interior) {
+            const cplx<T> *sc = reinterpret_cast<const cplx<T> *>(ring + (size_t)buf * SLABB) + (centre ? 0 : 26 * kNR) + row;
+            cplx<T> c[14];
+            if (run) {
+#pragma unroll
+                for (int t = 0; t < 14; ++t) c[t] = sc[sg * t * kNR];
+                if (!centre) c[13] = mk<T>(T(0), T(0));
 #pragma unroll
                 for (int kk = 0; kk < RPT; ++kk)
                     if (mine & (1u << kk))
-                        row_project_c<T, kPX, kPY>(sx + (size_t)(r0 + kk) * kNB, c, m, bv[kk], inv, w, lc);
-            } else {
-                T cr[27];
-                if (sp.adj) interior_coefs<T, true, kPX, kPY>(op, swr, lc, cr);
-                else interior_coefs<T, false, kPX, kPY>(op, swr, lc, cr);
+                        part[kk] = half_gather<T, kPX, kPY>(sx + (size_t)(r0 + kk) * kNB, c, xv[kk], lc, sg);
+            }
+            // neighbours outside the grid keep reading zero: a row on a face of the grid scatters to its
+            // inside neighbours only
+            uint32_t m = 0x7ffffffu;
+            if (edge_block && (i == 0 || j == 0 || k == 0 || i == op.nx - 1 || j == op.ny - 1 || k == op.nz - 1))
+                m = inside_mask(i, j, k, op.nx, op.ny, op.nz);
+            if (!centre) m = (__brev(m) >> 5) & 0x1fffu;  // bit t: offset 26 - t, no centre
+#pragma unroll
+            for (int kk = 0; kk < RPT; ++kk) {
+                const cplx<T> d = project(kk);
+                if (run && (mine & (1u << kk)))
+                    half_scatter<T, kPX, kPY>(sx + (size_t)(r0 + kk) * kNB, c, xv[kk], d, m, lc, sg);
+            }
+        } else {
+            T cr[14];
+            if (run) {
+                if (sp.adj) half_interior_coefs<T, true, kPX, kPY>(op, swr, lc, sg, centre, cr);
+                else half_interior_coefs<T, false, kPX, kPY>(op, swr, lc, sg, centre, cr);
 #pragma unroll
                 for (int kk = 0; kk < RPT; ++kk)
-                    if (mine & (1u << kk)) row_project_r<T, kPX, kPY>(sx + (size_t)(r0 + kk) * kNB, cr, bv[kk], inv, w, lc);
+                    if (mine & (1u << kk))
+                        part[kk] = half_gather_r<T, kPX, kPY>(sx + (size_t)(r0 + kk) * kNB, cr, xv[kk], lc, sg);
+            }
+#pragma unroll
+            for (int kk = 0; kk < RPT; ++kk) {
+                const cplx<T> d = project(kk);
+                if (run && (mine & (1u << kk)))
+                    half_scatter_r<T, kPX, kPY>(sx + (size_t)(r0 + kk) * kNB, cr, xv[kk], d, centre, lc, sg);
             }
         }
         if (__syncthreads_or(!ok)) {
@@ -366,7 +400,7 @@ int launch_b8(const B8Prob<T> *probs, const int *starts, int nprob, long long nc
                                           (int)smem));
         attr_set = true;
     }
-    sweep_b8_kernel<T, R, RPT, S><<<(unsigned)nctas, kNR * R / RPT, smem, st>>>(
+    sweep_b8_kernel<T, R, RPT, S><<<(unsigned)nctas, 2 * kNR * R / RPT, smem, st>>>(
         probs, starts, nprob, x, b, w, active, par, backward, nsteps, err, limit_ns, selftest);
     return H3D_OK;
 }

@@ -196,71 +196,90 @@ __device__ __forceinline__ void block_row_stored(const Op<T> &op, cplx<T> *bx, c
 #undef H3D_SS
 }
 
-// Row projections with the coefficients already in registers, so that one thread can project
-// the same row for several right-hand sides from one load of its coefficients.
-//   row_project_c: complex coefficients; the scatter skips the neighbours outside m
-//   row_project_r: real coefficients of an interior row (nothing outside the grid)
-// The gathered values stay in registers for the scatter (the footprint is the row's alone
-// within its colour).
+// A row projection by two lanes (16 apart in the warp): lane h = 0 holds offsets t = 0 .. 13, lane
+// h = 1 offsets 26 .. 14, the mirror images, so that both run the same code with a sign (sg = 1 or
+// -1); the centre t = 13 belongs to h = 0.  Slot t of the lane is offset t or 26 - t.
+//   half_gather   partial a.x over the lane's slots; the gathered values stay in xv for the scatter
+//                 (the footprint is the row's alone within its colour)
+//   half_scatter  x += d conj(a) on the lane's slots with bit t of m set
+// Real coefficients (interior rows): the same with cr.
+#define H3D_FOR_14(M)                                                                          \
+    M(0, -1, -1, -1) M(1, 0, -1, -1) M(2, 1, -1, -1) M(3, -1, 0, -1) M(4, 0, 0, -1)          \
+    M(5, 1, 0, -1) M(6, -1, 1, -1) M(7, 0, 1, -1) M(8, 1, 1, -1) M(9, -1, -1, 0)             \
+    M(10, 0, -1, 0) M(11, 1, -1, 0) M(12, -1, 0, 0) M(13, 0, 0, 0)
+
 template <typename T, int PX, int PY>
-__device__ __forceinline__ void row_project_c(cplx<T> *bx, const cplx<T> (&c)[27], uint32_t m, cplx<T> bv, T inv,
-                                              T w, int lc)
+__device__ __forceinline__ cplx<T> half_gather(const cplx<T> *bx, const cplx<T> (&c)[14], cplx<T> (&xv)[14], int lc, int sg)
 {
-    cplx<T> xv[27];
-    const cplx<T> z = mk<T>(T(0), T(0));
-    CSum<T> acc[3] = {csum_init(z), csum_init(z), csum_init(z)};
-#define H3D_GP(t, dx, dy, dz)                                                                  \
+    CSum<T> acc[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) acc[q] = csum_init(mk<T>(T(0), T(0)));
+#define H3D_HG(t, dx, dy, dz)                                                                  \
     {                                                                                          \
-        xv[t] = bx[lc + dx + PX * (dy + PY * dz)];                                             \
-        csum_mac(acc[dz + 1], c[t], xv[t]);                                                    \
+        xv[t] = bx[lc + sg * (dx + PX * (dy + PY * dz))];                                      \
+        csum_mac(acc[t % 3], c[t], xv[t]);                                                     \
     }
-    H3D_FOR_27(H3D_GP)
-#undef H3D_GP
-    const cplx<T> atx = cadd(cadd(csum_value(acc[0]), csum_value(acc[1])), csum_value(acc[2]));
-    const Scat<T> sd = scat_of((w * inv) * (bv - atx));
-#define H3D_SP(t, dx, dy, dz)                                                                  \
+    H3D_FOR_14(H3D_HG)
+#undef H3D_HG
+    return cadd(cadd(csum_value(acc[0]), csum_value(acc[1])), csum_value(acc[2]));
+}
+
+template <typename T, int PX, int PY>
+__device__ __forceinline__ void half_scatter(cplx<T> *bx, const cplx<T> (&c)[14], const cplx<T> (&xv)[14], cplx<T> d,
+                                             uint32_t m, int lc, int sg)
+{
+    const Scat<T> sd = scat_of(d);
+#define H3D_HS(t, dx, dy, dz)                                                                  \
     if (m & (1u << t)) {                                                                       \
         cplx<T> o = xv[t];                                                                     \
         scat_mac(o, sd, c[t]);                                                                 \
-        bx[lc + dx + PX * (dy + PY * dz)] = o;                                                 \
+        bx[lc + sg * (dx + PX * (dy + PY * dz))] = o;                                          \
     }
-    H3D_FOR_27(H3D_SP)
-#undef H3D_SP
+    H3D_FOR_14(H3D_HS)
+#undef H3D_HS
 }
 
 template <typename T, int PX, int PY>
-__device__ __forceinline__ void row_project_r(cplx<T> *bx, const T (&cr)[27], cplx<T> bv, T inv, T w, int lc)
+__device__ __forceinline__ cplx<T> half_gather_r(const cplx<T> *bx, const T (&cr)[14], cplx<T> (&xv)[14], int lc, int sg)
 {
-    cplx<T> xv[27];
-    cplx<T> acc[3] = {mk<T>(T(0), T(0)), mk<T>(T(0), T(0)), mk<T>(T(0), T(0))};
-#define H3D_GR(t, dx, dy, dz)                                                                  \
+    cplx<T> acc[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) acc[q] = mk<T>(T(0), T(0));
+#define H3D_HG(t, dx, dy, dz)                                                                  \
     {                                                                                          \
-        xv[t] = bx[lc + dx + PX * (dy + PY * dz)];                                             \
-        fma_rc(acc[dz + 1], cr[t], xv[t]);                                                     \
+        xv[t] = bx[lc + sg * (dx + PX * (dy + PY * dz))];                                      \
+        fma_rc(acc[t % 3], cr[t], xv[t]);                                                      \
     }
-    H3D_FOR_27(H3D_GR)
-#undef H3D_GR
-    const cplx<T> atx = cadd(cadd(acc[0], acc[1]), acc[2]);
-    const cplx<T> d = (w * inv) * (bv - atx);
-#define H3D_SR(t, dx, dy, dz)                                                                  \
-    {                                                                                          \
-        cplx<T> o = xv[t];                                                                     \
-        fma_rc(o, cr[t], d);                                                                   \
-        bx[lc + dx + PX * (dy + PY * dz)] = o;                                                 \
-    }
-    H3D_FOR_27(H3D_SR)
-#undef H3D_SR
+    H3D_FOR_14(H3D_HG)
+#undef H3D_HG
+    return cadd(cadd(acc[0], acc[1]), acc[2]);
 }
 
-// The 27 real coefficients of an interior row (all PML values 1, real wavenumber) from the
-// wavenumber box: K_t - WM_t wn (Helm3d_27pt.h:676-825 with xi = 1).
-template <typename T, bool ADJ, int PX, int PY>
-__device__ __forceinline__ void interior_coefs(const Op<T> &op, const T *swr, int lc, T (&cr)[27])
+template <typename T, int PX, int PY>
+__device__ __forceinline__ void half_scatter_r(cplx<T> *bx, const T (&cr)[14], const cplx<T> (&xv)[14], cplx<T> d,
+                                               bool centre, int lc, int sg)
 {
-    auto wnr = [&](int dx, int dy, int dz) { return swr[lc + dx + PX * (dy + PY * dz)]; };
+#define H3D_HS(t, dx, dy, dz)                                                                  \
+    if (t < 13 || centre) {                                                                    \
+        cplx<T> o = xv[t];                                                                     \
+        fma_rc(o, cr[t], d);                                                                   \
+        bx[lc + sg * (dx + PX * (dy + PY * dz))] = o;                                          \
+    }
+    H3D_FOR_14(H3D_HS)
+#undef H3D_HS
+}
+
+// The lane's 14 real coefficients of an interior row (all PML values 1, real wavenumber) from the
+// wavenumber box: K_t - WM_t wn (Helm3d_27pt.h:676-825 with xi = 1; K and WM are the same for t and
+// 26 - t); centre: the lane has the centre offset, else its slot is 0.
+template <typename T, bool ADJ, int PX, int PY>
+__device__ __forceinline__ void half_interior_coefs(const Op<T> &op, const T *swr, int lc, int sg, bool centre, T (&cr)[14])
+{
+    auto wnr = [&](int dx, int dy, int dz) { return swr[lc + sg * (dx + PX * (dy + PY * dz))]; };
 #define H3D_CIR(t, dx, dy, dz) cr[t] = coef_int<t, dx, dy, dz, T, ADJ>(op, wnr);
-    H3D_FOR_27(H3D_CIR)
+    H3D_FOR_14(H3D_CIR)
 #undef H3D_CIR
+    if (!centre) cr[13] = T(0);
 }
 
 }  // namespace h3d
