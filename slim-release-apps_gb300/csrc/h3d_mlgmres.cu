@@ -18,13 +18,16 @@
 // inner solver) owns its Krylov basis, a partial-sum buffer and a small state block
 // (FgState) in device memory.  An Arnoldi step is three launches: the matvec, the k inner
 // products V^H w (per-CTA partial sums), and the orthogonalisation w -= V h fused with the final
-// sum of those partials and with ||w||^2 partials, whose last CTA applies the previous Givens
-// rotations to the new Hessenberg column, forms the next rotation and updates the rotated
-// right-hand side and the quasi-residual.  The basis is kept unnormalised with a scale per
+// sum of those partials and with ||w||^2 partials.  The step's Givens update (the previous rotations
+// on the new Hessenberg column, the next rotation, the rotated right-hand side and the
+// quasi-residual: a dependent chain of some 100 FP64 instructions, about 5 us) runs beside the next
+// step's inner products, in a CTA of its own, or ends the cycle together with the back substitution; the
+// preconditioned instances, whose next step the host decides on, run it in the last CTA of the
+// orthogonalisation.  The basis is kept unnormalised with a scale per
 // vector in the unpreconditioned instances; the preconditioned ones (whose basis vectors feed
 // the V-cycle) add a fourth launch, the scaling V(:,k+1) = w / ||w||.  The Givens update gives
 // the least-squares residual norm of FGMRES.m:111-113 without a host round trip; the solution y
-// is back-substituted once per cycle, in the update of x.  Every kernel after the matvec reads
+// is back-substituted once per cycle.  Every kernel after the matvec reads
 // a flag of the state block (the step runs / the cycle runs) and returns at once when it is
 // clear, so the host enqueues a whole unpreconditioned cycle without waiting: it
 // synchronises once per cycle there, and before each step of a preconditioned instance (to
@@ -65,6 +68,7 @@ struct FgState {
     double rnormr0;             // 1 / normr0
     double sv[kMaxM];           // basis vector j = sv[j] x stored vector j (1 when stored normalised)
     int ticket;                 // CTAs of the current orthogonalisation launch that have finished
+    int pend;                   // steps orthogonalised whose Givens update is outstanding: j + 1, or 0
     double gres;                // |g(k+1)|: the current quasi-residual norm (before / normr0)
     double cs[kMaxM];           // Givens rotations: cosines (real) ...
     cplx<double> sn[kMaxM];     // ... and sines
@@ -75,6 +79,14 @@ struct FgState {
 };
 
 __device__ __forceinline__ bool closed(const int *gate) { return gate && *gate == 0; }
+
+// First thing in every kernel here: let the next launch set up early, and wait for the launch before
+// (both do nothing in an ordinary launch).
+__device__ __forceinline__ void fg_begin()
+{
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
 
 // Block-wide sum of two per-thread values kept in the field's precision T: warp shuffles in T,
 // the eight per-warp results added in FP64 by thread 0 in a fixed order (valid there).  GB300
@@ -112,6 +124,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThr) fg_copy_kernel(const cplx<T> *__restrict__ b, cplx<T> *__restrict__ r,
                                                        cplx<T> *__restrict__ x, long long n, double *part)
 {
+    fg_begin();
     T s = 0;
     for (long long e = blockIdx.x * (long long)kThr + threadIdx.x; e < n; e += (long long)gridDim.x * kThr) {
         const cplx<T> v = b[e];
@@ -128,6 +141,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThr) fg_sub_kernel(const cplx<T> *__restrict__ b, const cplx<T> *ax, cplx<T> *r,
                                                       long long n, double *part, const int *gate)
 {
+    fg_begin();
     if (closed(gate)) return;
     T s = 0;
     for (long long e = blockIdx.x * (long long)kThr + threadIdx.x; e < n; e += (long long)gridDim.x * kThr) {
@@ -145,6 +159,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThr) fg_scale_kernel(const cplx<T> *__restrict__ src, cplx<T> *__restrict__ dst,
                                                         long long n, const double *rcp, const int *gate)
 {
+    fg_begin();
     if (closed(gate)) return;
     const T d = (T)*rcp;
     for (long long e = blockIdx.x * (long long)kThr + threadIdx.x; e < n; e += (long long)gridDim.x * kThr) {
@@ -157,19 +172,34 @@ __global__ void __launch_bounds__(kThr) fg_scale_kernel(const cplx<T> *__restric
 // warp) so that kU x (vectors) independent loads are in flight before the arithmetic.
 constexpr int kU = 4;
 
+__device__ void givens_step(FgState *st, const double *part, int nparts, int j, int m, double tol, double *hist,
+                            int lazy);
+
 // Per-CTA partials of h_j = V_j^H w, j < nv <= MV: part[j * gridDim.x + cta].
 // Stored vector 0 is u0, vector j >= 1 is V + j n (the unpreconditioned instances keep vector 0
 // in their residual buffer).
+// The last CTA (blockIdx.x = nd) runs the Givens update of the step before instead, when it is
+// outstanding: the inner products do not need it, the orthogonalisation after them does.
 template <typename T, int MV>
 __global__ void __launch_bounds__(kThr) fg_dots_kernel(const cplx<T> *__restrict__ u0, const cplx<T> *__restrict__ V,
                                                        int nv, const cplx<T> *__restrict__ w, long long n,
-                                                       double2 *__restrict__ part, const int *gate)
+                                                       double2 *__restrict__ part, const int *gate, FgState *st,
+                                                       const double *npart, int m, double tol, double *hist)
 {
+    fg_begin();
+    const int nd = gridDim.x - 1;
+    if ((int)blockIdx.x == nd) {
+        const int pend = st->pend;
+        if (pend == 0) return;
+        givens_step(st, npart, nd, pend - 1, m, tol, hist, 1);
+        if (threadIdx.x == 0) st->pend = 0;
+        return;
+    }
     if (closed(gate)) return;
     cplx<T> acc[MV];
 #pragma unroll
     for (int j = 0; j < MV; ++j) acc[j] = mk<T>(0, 0);
-    const long long stride = (long long)gridDim.x * kThr;
+    const long long stride = (long long)nd * kThr;
     long long e = blockIdx.x * (long long)kThr + threadIdx.x;
     for (; e + (kU - 1) * stride < n; e += kU * stride) {
         cplx<T> wv[kU];
@@ -197,7 +227,7 @@ __global__ void __launch_bounds__(kThr) fg_dots_kernel(const cplx<T> *__restrict
     for (int j = 0; j < MV; ++j) {
         if (j < nv) {
             const double2 t = block_sum_t<T>(acc[j].re, acc[j].im);
-            if (threadIdx.x == 0) part[(long long)j * gridDim.x + blockIdx.x] = t;
+            if (threadIdx.x == 0) part[(long long)j * nd + blockIdx.x] = t;
         }
     }
 }
@@ -216,8 +246,10 @@ __device__ double sum_parts_cg(const double *part, int nparts)
 // new rotation needs only reciprocal square roots (FP64 divisions and square roots are long
 // dependent sequences on this GPU): c = |a| / r, s = (a / |a|) ||w|| / r, r = sqrt(|a|^2 +
 // ||w||^2), and the quasi-residual |g(j+2)| = |s| |g(j+1)| follows without a square root.
-// Run by every thread of the CTA that finishes the orthogonalisation last (fg_orth_kernel); the
-// state it reads is copied to shared memory by all its threads at once.
+// Run by every thread of one CTA: the one that finishes the orthogonalisation last (preconditioned
+// instances, whose next step the host decides on), an extra one of the next step's inner products, or
+// the one that ends the cycle (fg_finish_kernel); the state it reads is copied to shared memory by
+// all its threads at once.
 // hist (optional): the quasi-residual history, hist[nhst] written after each step.
 // lazy: the next basis vector is kept as w itself with scale 1 / ||w||.
 __device__ void givens_step(FgState *st, const double *part, int nparts, int j, int m, double tol, double *hist,
@@ -308,16 +340,17 @@ __device__ __forceinline__ void csub_mul(cplx<T> &a, cplx<T> v, cplx<T> h)
 // CTA in the same fixed order, so all agree; CTA 0 stores h in the state) and scaled by the
 // stored vectors' factors: the basis vector j is sv[j] times stored vector j, win = A (stored
 // vector k).  Per-CTA partials of ||wout||^2.  wout may be win.  nv <= MV.
-// The CTA that finishes last (a ticket counter in the state: every CTA publishes its partial,
+// tail: the CTA that finishes last (a ticket counter in the state: every CTA publishes its partial,
 // fences, then takes a ticket; no CTA waits for another) runs the step's Givens update
-// (givens_step) for step j = nv - 1 and resets the counter.
+// (givens_step) for step j = nv - 1 and resets the counter.  Otherwise the update is left outstanding.
 template <typename T, int MV>
 __global__ void __launch_bounds__(kThr) fg_orth_kernel(const cplx<T> *__restrict__ u0, const cplx<T> *__restrict__ V,
                                                        int nv, const cplx<T> *win, cplx<T> *wout, long long n,
                                                        const double2 *__restrict__ dpart, int nparts, FgState *st,
-                                                       double *part, int m, double tol, double *hist, int lazy,
+                                                       double *part, int m, double tol, double *hist, int tail,
                                                        const int *gate)
 {
+    fg_begin();
     if (closed(gate)) return;
     __shared__ cplx<T> sh[kMaxM];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -328,9 +361,13 @@ __global__ void __launch_bounds__(kThr) fg_orth_kernel(const cplx<T> *__restrict
             re += v.x;
             im += v.y;
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            re += __shfl_down_sync(0xffffffffu, re, o);
-            im += __shfl_down_sync(0xffffffffu, im, o);
+        // lanes 0-15 sum the real parts, 16-31 the imaginary ones: half the FP64 additions
+        {
+            const bool hi = lane & 16;
+            double t = (hi ? im : re) + __shfl_xor_sync(0xffffffffu, hi ? re : im, 16);
+            for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            re = t;
+            im = __shfl_xor_sync(0xffffffffu, t, 16);
         }
         if (lane == 0) {
             const double f = st->sv[j] * st->sv[nv - 1];
@@ -379,6 +416,13 @@ __global__ void __launch_bounds__(kThr) fg_orth_kernel(const cplx<T> *__restrict
         s = fma(a.re, a.re, fma(a.im, a.im, s));
     }
     const double2 t = block_sum_t<T>(s, T(0));
+    if (!tail) {
+        if (threadIdx.x == 0) {
+            part[blockIdx.x] = t.x;
+            if (blockIdx.x == 0) st->pend = nv;
+        }
+        return;
+    }
     __shared__ int last;
     if (threadIdx.x == 0) {
         part[blockIdx.x] = t.x;
@@ -388,41 +432,59 @@ __global__ void __launch_bounds__(kThr) fg_orth_kernel(const cplx<T> *__restrict
     __syncthreads();
     if (!last) return;
     __threadfence();
-    givens_step(st, part, gridDim.x, nv - 1, m, tol, hist, lazy);
+    givens_step(st, part, gridDim.x, nv - 1, m, tol, hist, 0);
     if (threadIdx.x == 0) st->ticket = 0;
 }
 
-// x += sum_{j < k} B_j y_j over the steps of the cycle (FGMRES.m:117-121).  y = R \ g, the
-// least-squares solution of FGMRES.m:111 after the cycle's last step, is back-substituted here
-// (thread 0 of every CTA, from the rotated Hessenberg matrix) rather than after every step;
-// CTA 0 stores it in the state.
+// End of a cycle's steps, one CTA: the outstanding Givens update, then y = R \ g, the least-squares
+// solution of FGMRES.m:111 after the last step, back-substituted from the rotated Hessenberg matrix.
+__global__ void __launch_bounds__(kThr) fg_finish_kernel(FgState *st, const double *part, int nparts, int m, double tol,
+                                                         double *hist)
+{
+    fg_begin();
+    if (st->hd.live == 0) return;
+    const int pend = st->pend;
+    __syncthreads();
+    if (pend) givens_step(st, part, nparts, pend - 1, m, tol, hist, 1);
+    __syncthreads();
+    __shared__ cplx<double> sR[kMaxM * kMaxM], sg[kMaxM], sy[kMaxM];
+    const int kk = st->hd.k;
+    for (int q = threadIdx.x; q < kk * kMaxM; q += kThr) sR[q] = st->R[q];
+    if (threadIdx.x < kk) sg[threadIdx.x] = st->g[threadIdx.x];
+    // the reciprocals of the diagonal do not wait for one another
+    __shared__ double srd[kMaxM];
+    __syncthreads();
+    if (threadIdx.x < kk) {
+        const double dd = cabs2(sR[threadIdx.x * kMaxM + threadIdx.x]);
+        srd[threadIdx.x] = dd == 0.0 ? 0.0 : 1.0 / dd;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    st->pend = 0;
+    for (int i = kk - 1; i >= 0; --i) {
+        cplx<double> t = sg[i];
+        for (int l = i + 1; l < kk; ++l) t = t - sR[l * kMaxM + i] * sy[l];
+        sy[i] = srd[i] * (t * cconj(sR[i * kMaxM + i]));
+        st->y[i] = sy[i];
+    }
+}
+
+// x += sum_{j < k} B_j y_j over the steps of the cycle (FGMRES.m:117-121), y from fg_finish_kernel.
 // Stored vector 0 is u0, vector j >= 1 is B + j n; with scaled != 0 the basis vector j is sv[j]
 // times the stored one.
 template <typename T>
 __global__ void __launch_bounds__(kThr) fg_xupd_kernel(cplx<T> *__restrict__ x, const cplx<T> *__restrict__ u0,
-                                                       const cplx<T> *__restrict__ B, long long n, FgState *st,
+                                                       const cplx<T> *__restrict__ B, long long n, const FgState *st,
                                                        int scaled, const int *gate)
 {
+    fg_begin();
     if (closed(gate)) return;
-    __shared__ cplx<double> sR[kMaxM * kMaxM], sg[kMaxM], sy[kMaxM];
     __shared__ cplx<T> syt[kMaxM];
     const int kk = st->hd.k;
-    for (int q = threadIdx.x; q < kk * kMaxM; q += kThr) sR[q] = st->R[q];
-    if (threadIdx.x < kk) sg[threadIdx.x] = st->g[threadIdx.x];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = kk - 1; i >= 0; --i) {
-            cplx<double> t = sg[i];
-            for (int l = i + 1; l < kk; ++l) t = t - sR[l * kMaxM + i] * sy[l];
-            const cplx<double> d = sR[i * kMaxM + i];
-            const double dd = cabs2(d);
-            sy[i] = dd == 0.0 ? mk<double>(0, 0) : (1.0 / dd) * (t * cconj(d));
-        }
-        for (int i = 0; i < kk; ++i) {
-            const double f = scaled ? st->sv[i] : 1.0;
-            syt[i] = mk<T>((T)(f * sy[i].re), (T)(f * sy[i].im));
-            if (blockIdx.x == 0) st->y[i] = sy[i];
-        }
+    if (threadIdx.x < kk) {
+        const double f = scaled ? st->sv[threadIdx.x] : 1.0;
+        const cplx<double> yv = st->y[threadIdx.x];
+        syt[threadIdx.x] = mk<T>((T)(f * yv.re), (T)(f * yv.im));
     }
     __syncthreads();
     const long long stride = (long long)gridDim.x * kThr;
@@ -481,6 +543,7 @@ __device__ __forceinline__ bool cycles_left(int it, int m, long long maxit)
 __global__ void __launch_bounds__(kThr) fg_norm_kernel(FgState *st, const double *part, int nparts, int first,
                                                        double tol, int m, long long maxit, int lazy)
 {
+    fg_begin();
     if (!first && st->hd.live == 0) return;
     const double nr = sqrt(sum_parts(part, nparts));
     if (threadIdx.x != 0) return;
@@ -511,6 +574,7 @@ __global__ void __launch_bounds__(kThr) fg_norm_kernel(FgState *st, const double
         st->rnormr0 = nr != 0.0 ? 1.0 / nr : 0.0;
         st->ticket = 0;
     }
+    st->pend = 0;
     h.k = 0;
     h.go = h.live;
     st->g[0] = mk<double>(nr, 0.0);
@@ -588,6 +652,7 @@ struct Run {                    // per-call context
     cudaStream_t s = nullptr;
     bool adj = false;
     int64_t launches = 0, syncs = 0;
+    long long before = -1;      // CTAs of the launch before on the stream, -1: not one to overlap with
     FgHead *hh = nullptr;       // pinned copy of a state head
 
     int fetch(const FgState *st)
@@ -595,6 +660,7 @@ struct Run {                    // per-call context
         H3D_CUDA_TRY(cudaMemcpyAsync(hh, &st->hd, sizeof(FgHead), cudaMemcpyDeviceToHost, s));
         H3D_CUDA_TRY(cudaStreamSynchronize(s));
         ++syncs;
+        before = -1;
         return H3D_OK;
     }
     unsigned blocks(long long n) const
@@ -608,7 +674,33 @@ struct Run {                    // per-call context
     do {                                     \
         __VA_ARGS__;                         \
         ++R.launches;                        \
+        R.before = -1;                       \
         H3D_CUDA_TRY(cudaGetLastError());    \
+    } while (0)
+
+// A launch of a kernel that begins with fg_begin: set up while the launch before still runs, where the
+// two together leave every CTA an SM of its own (the coarse levels, whose launches take a few
+// microseconds each; larger grids would crowd the SMs that free up first).
+template <typename... KA, typename... A>
+int fg_launch(Run &R, unsigned grid, void (*kern)(KA...), A... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kThr);
+    cfg.stream = R.s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = R.before > 0 && R.before + (long long)grid <= device_sms() ? 1 : 0;
+    H3D_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...));
+    R.before = grid;
+    ++R.launches;
+    return H3D_OK;
+}
+#define H3D_FG(...)                                        \
+    do {                                                   \
+        if ((rc = fg_launch(R, __VA_ARGS__))) return rc;   \
     } while (0)
 
 // FGMRES.m on one instance: x (in/out; zero_x = the initial guess is zero, FGMRES.m:65-67).
@@ -622,17 +714,20 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
     const int m = I.m;
     const unsigned nb = (unsigned)I.nparts;
     int rc;
-    if (zero_x) {
-        H3D_ML_LAUNCH((fg_copy_kernel<T><<<nb, kThr, 0, R.s>>>(b, I.r, x, n, I.part)));
-    } else {
-        if ((rc = launch_mvp<T>(op, x, I.w, 1, R.adj, false, R.s))) return rc;
+    auto matvec = [&](const cplx<T> *in, cplx<T> *out) -> int {
         ++R.launches;
-        H3D_ML_LAUNCH((fg_sub_kernel<T><<<nb, kThr, 0, R.s>>>(b, I.w, I.r, n, I.part, nullptr)));
+        return launch_mvp<T>(op, in, out, 1, R.adj, false, R.s, &R.before);
+    };
+    if (zero_x) {
+        H3D_FG(nb, fg_copy_kernel<T>, b, I.r, x, n, I.part);
+    } else {
+        if ((rc = matvec(x, I.w))) return rc;
+        H3D_FG(nb, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, nullptr);
     }
     // Unpreconditioned instances keep their basis unnormalised (each stored vector with its scale
     // in the state): no separate scaling pass per step; vector 0 is the residual buffer itself.
     const int lazy = pre ? 0 : 1;
-    H3D_ML_LAUNCH((fg_norm_kernel<<<1, kThr, 0, R.s>>>(I.st, I.part, I.nparts, 1, tol, m, maxit, lazy)));
+    H3D_FG(1u, fg_norm_kernel, I.st, I.part, I.nparts, 1, tol, m, maxit, lazy);
     int *live = &I.st->hd.live, *go = &I.st->hd.go;
     const cplx<T> *u0 = lazy ? I.r : I.V;
     cplx<T> *basis = pre ? I.Z : I.V;
@@ -641,7 +736,7 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
             if ((rc = R.fetch(I.st))) return rc;
             if (!R.hh->live) break;
         }
-        if (!lazy) H3D_ML_LAUNCH((fg_scale_kernel<T><<<nb, kThr, 0, R.s>>>(I.r, I.V, n, &I.st->rbeta, live)));
+        if (!lazy) H3D_FG(nb, fg_scale_kernel<T>, I.r, I.V, n, &I.st->rbeta, live);
         for (int j = 0; j < m; ++j) {
             const cplx<T> *vj = j == 0 ? u0 : I.V + (long long)j * n;
             if (pre) {
@@ -653,36 +748,26 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
                 if ((rc = (*pre)(vj, zj))) return rc;
                 vj = zj;
             }
-            if ((rc = launch_mvp<T>(op, vj, I.w, 1, R.adj, false, R.s))) return rc;
-            ++R.launches;
+            if ((rc = matvec(vj, I.w))) return rc;
             // the orthogonalised vector: straight into the next basis slot (lazy), else into w
             cplx<T> *wout = (lazy && j + 1 < m) ? I.V + (long long)(j + 1) * n : I.w;
-            if (j < 4) {
-                H3D_ML_LAUNCH((fg_dots_kernel<T, 4><<<nb, kThr, 0, R.s>>>(u0, I.V, j + 1, I.w, n, I.dpart, go)));
-                H3D_ML_LAUNCH((fg_orth_kernel<T, 4><<<nb, kThr, 0, R.s>>>(u0, I.V, j + 1, I.w, wout, n, I.dpart,
-                                                                          I.nparts, I.st, I.part, m, tol, I.hist,
-                                                                          lazy, go)));
-            } else if (j < 8) {
-                H3D_ML_LAUNCH((fg_dots_kernel<T, 8><<<nb, kThr, 0, R.s>>>(u0, I.V, j + 1, I.w, n, I.dpart, go)));
-                H3D_ML_LAUNCH((fg_orth_kernel<T, 8><<<nb, kThr, 0, R.s>>>(u0, I.V, j + 1, I.w, wout, n, I.dpart,
-                                                                          I.nparts, I.st, I.part, m, tol, I.hist,
-                                                                          lazy, go)));
-            } else {
-                H3D_ML_LAUNCH((fg_dots_kernel<T, kMaxM><<<nb, kThr, 0, R.s>>>(u0, I.V, j + 1, I.w, n, I.dpart, go)));
-                H3D_ML_LAUNCH((fg_orth_kernel<T, kMaxM><<<nb, kThr, 0, R.s>>>(u0, I.V, j + 1, I.w, wout, n, I.dpart,
-                                                                              I.nparts, I.st, I.part, m, tol, I.hist,
-                                                                          lazy, go)));
-            }
-            if (!lazy && j + 1 < m)
-                H3D_ML_LAUNCH((fg_scale_kernel<T><<<nb, kThr, 0, R.s>>>(I.w, I.V + (long long)(j + 1) * n, n,
-                                                                        &I.st->rhn, go)));
+            auto step = [&](auto dots, auto orth) -> int {
+                H3D_FG(nb + 1, dots, u0, I.V, j + 1, I.w, n, I.dpart, go, I.st, I.part, m, tol, I.hist);
+                H3D_FG(nb, orth, u0, I.V, j + 1, I.w, wout, n, I.dpart, I.nparts, I.st, I.part, m, tol, I.hist,
+                       pre ? 1 : 0, go);
+                return H3D_OK;
+            };
+            if (j < 4) rc = step(fg_dots_kernel<T, 4>, fg_orth_kernel<T, 4>);
+            else if (j < 8) rc = step(fg_dots_kernel<T, 8>, fg_orth_kernel<T, 8>);
+            else rc = step(fg_dots_kernel<T, kMaxM>, fg_orth_kernel<T, kMaxM>);
+            if (rc) return rc;
+            if (!lazy && j + 1 < m) H3D_FG(nb, fg_scale_kernel<T>, I.w, I.V + (long long)(j + 1) * n, n, &I.st->rhn, go);
         }
-        H3D_ML_LAUNCH(
-            (fg_xupd_kernel<T><<<nb, kThr, 0, R.s>>>(x, pre ? I.Z : u0, basis, n, I.st, lazy, live)));
-        if ((rc = launch_mvp<T>(op, x, I.w, 1, R.adj, false, R.s))) return rc;
-        ++R.launches;
-        H3D_ML_LAUNCH((fg_sub_kernel<T><<<nb, kThr, 0, R.s>>>(b, I.w, I.r, n, I.part, live)));
-        H3D_ML_LAUNCH((fg_norm_kernel<<<1, kThr, 0, R.s>>>(I.st, I.part, I.nparts, 0, tol, m, maxit, lazy)));
+        H3D_FG(1u, fg_finish_kernel, I.st, I.part, I.nparts, m, tol, I.hist);
+        H3D_FG(nb, fg_xupd_kernel<T>, x, pre ? I.Z : u0, basis, n, I.st, lazy, live);
+        if ((rc = matvec(x, I.w))) return rc;
+        H3D_FG(nb, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, live);
+        H3D_FG(1u, fg_norm_kernel, I.st, I.part, I.nparts, 0, tol, m, maxit, lazy);
     }
     if (last_fetch) return R.fetch(I.st);
     return H3D_OK;
@@ -757,6 +842,7 @@ struct Cycle {
                                     R.s)))
             return rcode;
         R.launches += 3;
+        R.before = -1;
         return H3D_OK;
     }
 
@@ -765,7 +851,7 @@ struct Cycle {
     {
         int rcode;
         if ((rcode = fgmres<T>(R, smooth[i], op[i], b, x, true, stol, sk, nullptr, false))) return rcode;
-        if ((rcode = launch_mvp<T>(op[i], x, res[i], 1, R.adj, false, R.s))) return rcode;
+        if ((rcode = launch_mvp<T>(op[i], x, res[i], 1, R.adj, false, R.s, &R.before))) return rcode;
         ++R.launches;
         const unsigned nb = (unsigned)smooth[i].nparts;
         H3D_ML_LAUNCH((fg_sub_kernel<T><<<nb, kThr, 0, R.s>>>(b, res[i], res[i], n[i], nullptr, nullptr)));

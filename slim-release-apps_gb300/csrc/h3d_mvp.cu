@@ -57,6 +57,9 @@ __global__ void __launch_bounds__(kMX *kMY) mvp_zmarch_kernel(Op<T> op, const cp
     __shared__ T swr[NEED_WN ? 2 : 1][NEED_WN ? kPN : 1];
     __shared__ T swi[NEED_WN && WNC ? 2 : 1][NEED_WN && WNC ? kPN : 1];
 
+    // the next launch may set up early; wait for the launch before (nothing in an ordinary launch)
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
     const int tid = threadIdx.x + kMX * threadIdx.y;
     const int s = blockIdx.z / nchunks, chunk = blockIdx.z % nchunks;
     const int kb = chunk * kz, ke = min(op.nz, kb + kz);
@@ -328,9 +331,27 @@ static bool use_flat(const Op<T> &op)
     return sizeof(T) == 8 && flat_smem<double, false, true>(op.nx) <= 96 * 1024;
 }
 
+// early: set up while the launch before still runs (it must let this one, and fill no SM it needs).
+template <typename... KA, typename... A>
+static int mvp_start(void (*kern)(KA...), dim3 grd, dim3 blk, size_t smem, bool early, cudaStream_t st, const A &...args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grd;
+    cfg.blockDim = blk;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = early ? 1 : 0;
+    H3D_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...));
+    return H3D_OK;
+}
+
 template <typename T, bool ADJ, bool DERIV, bool WNC, bool RESID>
 static int flat_launch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const cplx<T> *b, dim3 grd, int kz, int nch,
-                       double *part, cudaStream_t st)
+                       double *part, bool early, cudaStream_t st)
 {
     if constexpr (sizeof(T) == 8) {
         const size_t smem = flat_smem<T, ADJ, WNC>(op.nx);
@@ -339,14 +360,15 @@ static int flat_launch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const cplx
             H3D_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         auto aligned = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
         const int vec = aligned(x) && aligned(op.wn) && (!WNC || aligned(op.wni));
-        kern<<<grd, kFT, smem, st>>>(op, x, y, b, kz, nch, vec, part);
+        return mvp_start(kern, grd, dim3(kFT), smem, early, st, op, x, y, b, kz, nch, vec, part);
     }
     return H3D_OK;
 }
 
 template <typename T, bool RESID>
 static int zmarch_dispatch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const cplx<T> *b, int nrhs,
-                           bool adj, bool deriv, double *part, int parts, cudaStream_t st)
+                           bool adj, bool deriv, double *part, int parts, cudaStream_t st,
+                           long long *before = nullptr)
 {
     if ((long long)op.nx * op.ny >= (1LL << 31)) {
         set_error("a z plane of more than 2^31 - 1 points is not supported by the matvec");
@@ -369,9 +391,12 @@ static int zmarch_dispatch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const 
     const dim3 blk(kMX, kMY);
     const bool wnc = op.wni != nullptr;
     int rc = H3D_OK;
-#define H3D_ZM(A, D, W)                                                                        \
-    if (flat) rc = flat_launch<T, A, D, W, RESID>(op, x, y, b, grd, kz, nch, part, st);          \
-    else mvp_zmarch_kernel<T, A, D, W, RESID><<<grd, blk, 0, st>>>(op, x, y, b, kz, nch, part)
+    const long long ctas = (long long)grd.x * grd.y * grd.z;
+    const bool early = before && *before > 0 && *before + ctas <= device_sms();
+    if (before) *before = ctas;
+#define H3D_ZM(A, D, W)                                                                                   \
+    if (flat) rc = flat_launch<T, A, D, W, RESID>(op, x, y, b, grd, kz, nch, part, early, st);              \
+    else rc = mvp_start(mvp_zmarch_kernel<T, A, D, W, RESID>, grd, blk, 0, early, st, op, x, y, b, kz, nch, part)
     switch ((adj ? 4 : 0) + (deriv ? 2 : 0) + (wnc ? 1 : 0)) {
     case 0: H3D_ZM(false, false, false); break;
     case 1: H3D_ZM(false, false, true); break;
@@ -390,9 +415,9 @@ static int zmarch_dispatch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const 
 
 template <typename T>
 int launch_mvp(const Op<T> &op, const cplx<T> *x, cplx<T> *y, int nrhs, bool adj, bool deriv,
-               cudaStream_t st)
+               cudaStream_t st, long long *before)
 {
-    return zmarch_dispatch<T, false>(op, x, y, nullptr, nrhs, adj, deriv, nullptr, 0, st);
+    return zmarch_dispatch<T, false>(op, x, y, nullptr, nrhs, adj, deriv, nullptr, 0, st, before);
 }
 
 int mvp_residual_parts(const Op<double> &op, int nrhs)
@@ -412,7 +437,7 @@ int launch_residual(const Op<double> &op, const cplx<double> *b, const cplx<doub
     return zmarch_dispatch<double, true>(op, x, r, b, nrhs, adj, false, part, parts, st);
 }
 
-template int launch_mvp<double>(const Op<double> &, const cplx<double> *, cplx<double> *, int, bool, bool, cudaStream_t);
-template int launch_mvp<float>(const Op<float> &, const cplx<float> *, cplx<float> *, int, bool, bool, cudaStream_t);
+template int launch_mvp<double>(const Op<double> &, const cplx<double> *, cplx<double> *, int, bool, bool, cudaStream_t, long long *);
+template int launch_mvp<float>(const Op<float> &, const cplx<float> *, cplx<float> *, int, bool, bool, cudaStream_t, long long *);
 
 }  // namespace h3d

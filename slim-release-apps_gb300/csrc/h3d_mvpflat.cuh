@@ -94,6 +94,9 @@ __global__ void __launch_bounds__(kFT)
     C *sx = reinterpret_cast<C *>(fl_smem);
     T *sw = reinterpret_cast<T *>(sx + kFB * mp), *swi = sw + kFB * mp;
 
+    // the next launch may set up early; wait for the launch before (nothing in an ordinary launch)
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
     const int tid = threadIdx.x;
     const int s = blockIdx.y / nchunks, chunk = blockIdx.y % nchunks;
     const int kb = chunk * kz, ke = min(op.nz, kb + kz);
