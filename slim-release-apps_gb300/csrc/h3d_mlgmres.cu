@@ -232,12 +232,25 @@ __global__ void __launch_bounds__(kThr) fg_dots_kernel(const cplx<T> *__restrict
     }
 }
 
+// Block-wide FP64 sum of one value per thread (valid in thread 0): fixed order.
+__device__ double block_sum1(double a)
+{
+    __shared__ double sa[kThr / 32];
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if ((threadIdx.x & 31) == 0) sa[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (threadIdx.x >= kThr / 32) return 0.0;
+    a = sa[threadIdx.x];
+    for (int o = kThr / 64; o > 0; o >>= 1) a += __shfl_down_sync((1u << (kThr / 32)) - 1u, a, o);
+    return a;
+}
+
 // Sum of per-CTA partials written by other CTAs of the same launch (read through L2).
 __device__ double sum_parts_cg(const double *part, int nparts)
 {
     double s = 0.0;
     for (int p = threadIdx.x; p < nparts; p += kThr) s += __ldcg(part + p);
-    return block_sum_t<double>(s, 0.0).x;
+    return block_sum1(s);
 }
 
 // Step j of the cycle (0-based): H(1:j+1, j+1) = h, H(j+2, j+1) = ||w||; Givens rotations
@@ -266,12 +279,12 @@ __device__ void givens_step(FgState *st, const double *part, int nparts, int j, 
         const double2 v = __ldcg(reinterpret_cast<const double2 *>(st->h + threadIdx.x));
         sc[threadIdx.x] = mk<double>(v.x, v.y);
     }
+    const cplx<double> gj = st->g[j];
+    const double gres = st->gres, rnormr0 = st->rnormr0;
+    const int nhst = st->hd.nhst, it = st->hd.it;
     const double w2 = sum_parts_cg(part, nparts);  // ||w||^2 (synchronises the block)
     if (threadIdx.x != 0) return;
-    const cplx<double> gj = st->g[j];
-    const double gres = st->gres;
     FgHead &h = st->hd;
-    const double rnormr0 = st->rnormr0;
     const double rhn = w2 > 0.0 ? rsqrt(w2) : 0.0;
     const double hn = w2 * rhn;
     cplx<double> *c = sc;
@@ -318,10 +331,10 @@ __device__ void givens_step(FgState *st, const double *part, int nparts, int j, 
     st->hn = hn;
     st->rhn = rhn;
     if (j + 1 < kMaxM) st->sv[j + 1] = lazy ? rhn : 1.0;
-    const int nh = h.nhst + 1;
+    const int nh = nhst + 1;
     h.nhst = nh;
     if (hist) hist[nh] = q;
-    h.it += 1;
+    h.it = it + 1;
     h.k = j + 1;
     h.go = (q > tol && j + 1 < m) ? 1 : 0;
 }
@@ -449,8 +462,8 @@ __global__ void __launch_bounds__(kThr) fg_finish_kernel(FgState *st, const doub
     __syncthreads();
     __shared__ cplx<double> sR[kMaxM * kMaxM], sg[kMaxM], sy[kMaxM];
     const int kk = st->hd.k;
-    for (int q = threadIdx.x; q < kk * kMaxM; q += kThr) sR[q] = st->R[q];
-    if (threadIdx.x < kk) sg[threadIdx.x] = st->g[threadIdx.x];
+    for (int q = threadIdx.x; q < m * kMaxM; q += kThr) sR[q] = st->R[q];
+    if (threadIdx.x < m) sg[threadIdx.x] = st->g[threadIdx.x];
     // the reciprocals of the diagonal do not wait for one another
     __shared__ double srd[kMaxM];
     __syncthreads();
@@ -527,7 +540,7 @@ __device__ double sum_parts(const double *part, int nparts)
 {
     double s = 0.0;
     for (int p = threadIdx.x; p < nparts; p += kThr) s += part[p];
-    return block_sum_t<double>(s, 0.0).x;
+    return block_sum1(s);
 }
 
 __device__ __forceinline__ bool cycles_left(int it, int m, long long maxit)
@@ -625,6 +638,9 @@ struct Fg {                     // one FGMRES instance
     long long n = 0;
     int m = 0;
     bool pre = false;
+    // cycles enqueued between two reads of the state by the host (unpreconditioned instances): an
+    // instance that has stopped leaves x and r as they are, its further launches return at once
+    int ahead = 1;
     int nparts = 1;
     cplx<T> *V = nullptr, *Z = nullptr, *w = nullptr, *r = nullptr;
     double2 *dpart = nullptr;
@@ -703,12 +719,16 @@ int fg_launch(Run &R, unsigned grid, void (*kern)(KA...), A... args)
         if ((rc = fg_launch(R, __VA_ARGS__))) return rc;   \
     } while (0)
 
+// What a caller needs beside x: the state's head back on the host (the outer solve), the residual b - A x
+// in I.r, or nothing (then the residual after the last cycle, which decides nothing, is left out).
+enum FgTail { kFgHead, kFgResidual, kFgNone };
+
 // FGMRES.m on one instance: x (in/out; zero_x = the initial guess is zero, FGMRES.m:65-67).
 // pre: the flexible preconditioner z = P v (null = identity, the basis itself updates x).
-// last_fetch: read the state head back at the end (into R.hh).
+// tail: see FgTail (kFgHead reads the state head back at the end, into R.hh).
 template <typename T>
 int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool zero_x, double tol,
-           long long maxit, const Pre<T> *pre, bool last_fetch)
+           long long maxit, const Pre<T> *pre, FgTail tail)
 {
     const long long n = I.n;
     const int m = I.m;
@@ -732,17 +752,21 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
     const cplx<T> *u0 = lazy ? I.r : I.V;
     cplx<T> *basis = pre ? I.Z : I.V;
     for (long long c = 0; c < maxit; ++c) {
-        if (pre || c > 0) {
+        if (pre || (c > 0 && c % I.ahead == 0)) {
             if ((rc = R.fetch(I.st))) return rc;
             if (!R.hh->live) break;
         }
         if (!lazy) H3D_FG(nb, fg_scale_kernel<T>, I.r, I.V, n, &I.st->rbeta, live);
+        bool stopped = false;  // on the quasi-residual, as read by the host: no further cycle (FGMRES.m:88)
         for (int j = 0; j < m; ++j) {
             const cplx<T> *vj = j == 0 ? u0 : I.V + (long long)j * n;
             if (pre) {
                 if (j > 0) {
                     if ((rc = R.fetch(I.st))) return rc;
-                    if (!R.hh->go) break;
+                    if (!R.hh->go) {
+                        stopped = R.hh->hst <= tol;
+                        break;
+                    }
                 }
                 cplx<T> *zj = I.Z + (long long)j * n;
                 if ((rc = (*pre)(vj, zj))) return rc;
@@ -765,11 +789,13 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
         }
         H3D_FG(1u, fg_finish_kernel, I.st, I.part, I.nparts, m, tol, I.hist);
         H3D_FG(nb, fg_xupd_kernel<T>, x, pre ? I.Z : u0, basis, n, I.st, lazy, live);
+        if (tail == kFgNone && (stopped || c == maxit - 1)) break;
         if ((rc = matvec(x, I.w))) return rc;
         H3D_FG(nb, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, live);
+        if (tail == kFgResidual && c == maxit - 1) break;
         H3D_FG(1u, fg_norm_kernel, I.st, I.part, I.nparts, 0, tol, m, maxit, lazy);
     }
-    if (last_fetch) return R.fetch(I.st);
+    if (tail == kFgHead) return R.fetch(I.st);
     return H3D_OK;
 }
 
@@ -781,7 +807,7 @@ struct Cycle {
     long long n[kMaxLevels] = {};
     const h3d_ml_transfer *Rt = nullptr, *Pt = nullptr;
     Fg<T> smooth[kMaxLevels], coarse[kMaxLevels], bottom;
-    cplx<T> *res[kMaxLevels] = {}, *rc[kMaxLevels] = {}, *xc[kMaxLevels] = {};
+    cplx<T> *rc[kMaxLevels] = {}, *xc[kMaxLevels] = {};
     cplx<T> *t1 = nullptr, *t2 = nullptr;
     long long t1n = 0, t2n = 0;
     double stol = 1e-6, ctol = 0.5;
@@ -798,6 +824,8 @@ struct Cycle {
                 smooth[i].n = n[i];
                 smooth[i].m = k[1];
                 smooth[i].nparts = parts_for(n[i]);
+                // a smoother seldom meets its tolerance: the stream is not drained after each cycle
+                smooth[i].ahead = 4;
             }
             if (i >= 1) {
                 coarse[i].n = n[i];
@@ -815,7 +843,6 @@ struct Cycle {
         for (int i = 0; i < nl; ++i) {
             if (i < nl - 1) {
                 smooth[i].carve(a);
-                res[i] = a.take<cplx<T>>(n[i]);
             }
             if (i >= 1) {
                 coarse[i].carve(a);
@@ -850,23 +877,19 @@ struct Cycle {
     int vcycle(Run &R, int i, const cplx<T> *b, cplx<T> *x)
     {
         int rcode;
-        if ((rcode = fgmres<T>(R, smooth[i], op[i], b, x, true, stol, sk, nullptr, false))) return rcode;
-        if ((rcode = launch_mvp<T>(op[i], x, res[i], 1, R.adj, false, R.s, &R.before))) return rcode;
-        ++R.launches;
-        const unsigned nb = (unsigned)smooth[i].nparts;
-        H3D_ML_LAUNCH((fg_sub_kernel<T><<<nb, kThr, 0, R.s>>>(b, res[i], res[i], n[i], nullptr, nullptr)));
-        if ((rcode = transfer(R, Rt[i], res[i], rc[i + 1], false))) return rcode;
+        if ((rcode = fgmres<T>(R, smooth[i], op[i], b, x, true, stol, sk, nullptr, kFgResidual))) return rcode;
+        if ((rcode = transfer(R, Rt[i], smooth[i].r, rc[i + 1], false))) return rcode;  // b - A x
         Pre<T> pre;
         if (i + 1 == nl - 1)
             pre = [this, &R](const cplx<T> *v, cplx<T> *z) {
-                return fgmres<T>(R, bottom, op[nl - 1], v, z, true, ctol, ck, nullptr, false);
+                return fgmres<T>(R, bottom, op[nl - 1], v, z, true, ctol, ck, nullptr, kFgNone);
             };
         else
             pre = [this, &R, i](const cplx<T> *v, cplx<T> *z) { return vcycle(R, i + 1, v, z); };
-        if ((rcode = fgmres<T>(R, coarse[i + 1], op[i + 1], rc[i + 1], xc[i + 1], true, ctol, ck, &pre, false)))
+        if ((rcode = fgmres<T>(R, coarse[i + 1], op[i + 1], rc[i + 1], xc[i + 1], true, ctol, ck, &pre, kFgNone)))
             return rcode;
         if ((rcode = transfer(R, Pt[i], xc[i + 1], x, true))) return rcode;
-        return fgmres<T>(R, smooth[i], op[i], b, x, false, stol, sk, nullptr, false);
+        return fgmres<T>(R, smooth[i], op[i], b, x, false, stol, sk, nullptr, kFgNone);
     }
 };
 
@@ -1039,7 +1062,7 @@ extern "C" int h3d_mlgmres_solve(const h3d_ml_level *levels, int nlevels, const 
         pre = [&](const cplx<double> *v, cplx<double> *z) -> int { return c64.vcycle(R, 0, v, z); };
 
     rc = fgmres<double>(R, outer, op0, (const cplx<double> *)b, (cplx<double> *)x, false, o.tol, o.maxit,
-                        ml ? &pre : nullptr, true);
+                        ml ? &pre : nullptr, kFgHead);
     if (rc) return rc;
     if (hst) {
         hst[0] = 1.0;
