@@ -37,6 +37,7 @@
 //
 // The mixed precision of the Python front end carries over: the outer FGMRES in complex128,
 // the V-cycle (all levels, smoothers and coarse solves) in complex64 with FP64 inner products.
+#include <cfloat>
 #include <chrono>
 #include <cmath>
 #include <functional>
@@ -88,33 +89,27 @@ __device__ __forceinline__ void fg_begin()
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 
-// Block-wide sum of two per-thread values kept in the field's precision T: warp shuffles in T,
-// the eight per-warp results added in FP64 by thread 0 in a fixed order (valid there).  GB300
-// executes FP64 at a small fraction of its FP32 rate, so the complex64 cycle's vector kernels
-// form products and per-thread sums in FP32 (as a complex64 BLAS would) and leave FP64 to the
-// few values per CTA; the complex128 instances stay FP64 throughout.
-template <typename T>
-__device__ __forceinline__ double2 block_sum_t(T a, T b)
+// Sum over the block's warps of one FP64 value per warp and index: lane w of eight holds warp w's.
+__device__ __forceinline__ double warps_sum8(double v)
 {
-    __shared__ double sa[kThr / 32], sb[kThr / 32];
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-        sa[wid] = (double)a;
-        sb[wid] = (double)b;
-    }
+    for (int o = kThr / 64; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Block-wide sum of one per-thread value kept in precision T (valid in every thread of warp 0): warp
+// shuffles in T, the per-warp results added in FP64 in a fixed order.  GB300 executes FP64 at a small
+// fraction of its FP32 rate (a warp's FP64 instruction holds its scheduler's pipe for 64 cycles, however
+// few of its lanes are active), so the complex64 cycle's vector kernels form products and per-thread sums
+// in FP32 (as a complex64 BLAS would), leave FP64 to the few values per CTA, and add those as a tree
+// across lanes; the complex128 instances stay FP64 throughout.
+template <typename T>
+__device__ __forceinline__ double block_sum(T a)
+{
+    __shared__ double sa[kThr / 32];
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if ((threadIdx.x & 31) == 0) sa[threadIdx.x >> 5] = (double)a;
     __syncthreads();
-    double x = 0.0, y = 0.0;
-    if (threadIdx.x == 0)
-        for (int q = 0; q < kThr / 32; ++q) {
-            x += sa[q];
-            y += sb[q];
-        }
-    __syncthreads();
-    return make_double2(x, y);
+    return threadIdx.x < 32 ? warps_sum8(sa[threadIdx.x & (kThr / 32 - 1)]) : 0.0;
 }
 
 // ---- element kernels ----------------------------------------------------------------------
@@ -132,8 +127,8 @@ __global__ void __launch_bounds__(kThr) fg_copy_kernel(const cplx<T> *__restrict
         if (x) x[e] = mk<T>(0, 0);
         s = fma(v.re, v.re, fma(v.im, v.im, s));
     }
-    const double2 t = block_sum_t<T>(s, T(0));
-    if (threadIdx.x == 0) part[blockIdx.x] = t.x;
+    const double t = block_sum<T>(s);
+    if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
 // r = b - ax (r may alias ax); per-CTA partials of ||r||^2 when part is given.
@@ -150,8 +145,8 @@ __global__ void __launch_bounds__(kThr) fg_sub_kernel(const cplx<T> *__restrict_
         s = fma(v.re, v.re, fma(v.im, v.im, s));
     }
     if (!part) return;
-    const double2 t = block_sum_t<T>(s, T(0));
-    if (threadIdx.x == 0) part[blockIdx.x] = t.x;
+    const double t = block_sum<T>(s);
+    if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
 // dst = src * (*rcp): V(:,k) = w / ||w|| with the reciprocal formed once per step.
@@ -223,26 +218,35 @@ __global__ void __launch_bounds__(kThr) fg_dots_kernel(const cplx<T> *__restrict
         for (int j = 0; j < MV; ++j)
             if (j < nv) cmac_cb(acc[j], wv, (j == 0 ? u0 : V + (long long)j * n)[e]);
     }
+    // all the sums at once: warp sums in T, then eight lanes add each part's warp results
+    __shared__ double sw[MV * 2 * (kThr / 32)];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int j = 0; j < MV; ++j) {
-        if (j < nv) {
-            const double2 t = block_sum_t<T>(acc[j].re, acc[j].im);
-            if (threadIdx.x == 0) part[(long long)j * nd + blockIdx.x] = t;
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int j = 0; j < MV; ++j) {
+            if (j < nv) {
+                acc[j].re += __shfl_down_sync(0xffffffffu, acc[j].re, o);
+                acc[j].im += __shfl_down_sync(0xffffffffu, acc[j].im, o);
+            }
         }
     }
-}
-
-// Block-wide FP64 sum of one value per thread (valid in thread 0): fixed order.
-__device__ double block_sum1(double a)
-{
-    __shared__ double sa[kThr / 32];
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-    if ((threadIdx.x & 31) == 0) sa[threadIdx.x >> 5] = a;
+    if (lane == 0) {
+#pragma unroll
+        for (int j = 0; j < MV; ++j) {
+            if (j < nv) {
+                sw[(2 * j) * (kThr / 32) + wid] = (double)acc[j].re;
+                sw[(2 * j + 1) * (kThr / 32) + wid] = (double)acc[j].im;
+            }
+        }
+    }
     __syncthreads();
-    if (threadIdx.x >= kThr / 32) return 0.0;
-    a = sa[threadIdx.x];
-    for (int o = kThr / 64; o > 0; o >>= 1) a += __shfl_down_sync((1u << (kThr / 32)) - 1u, a, o);
-    return a;
+    static_assert(MV * 2 * (kThr / 32) <= kThr, "one thread per warp result");
+    if (wid * 32 >= nv * 2 * (kThr / 32)) return;  // whole warps: two vectors each
+    const int e2 = threadIdx.x, jc = e2 / (kThr / 32);
+    const double v = warps_sum8(jc < 2 * nv ? sw[e2] : 0.0);
+    if (jc < 2 * nv && (e2 & (kThr / 32 - 1)) == 0)
+        reinterpret_cast<double *>(part + (long long)(jc >> 1) * nd + blockIdx.x)[jc & 1] = v;
 }
 
 // Sum of per-CTA partials written by other CTAs of the same launch (read through L2).
@@ -250,7 +254,7 @@ __device__ double sum_parts_cg(const double *part, int nparts)
 {
     double s = 0.0;
     for (int p = threadIdx.x; p < nparts; p += kThr) s += __ldcg(part + p);
-    return block_sum1(s);
+    return block_sum<double>(s);
 }
 
 // Step j of the cycle (0-based): H(1:j+1, j+1) = h, H(j+2, j+1) = ||w||; Givens rotations
@@ -261,69 +265,86 @@ __device__ double sum_parts_cg(const double *part, int nparts)
 // ||w||^2), and the quasi-residual |g(j+2)| = |s| |g(j+1)| follows without a square root.
 // Run by every thread of one CTA: the one that finishes the orthogonalisation last (preconditioned
 // instances, whose next step the host decides on), an extra one of the next step's inner products, or
-// the one that ends the cycle (fg_finish_kernel); the state it reads is copied to shared memory by
-// all its threads at once.
+// the one that ends the cycle (fg_finish_kernel).  One warp does the arithmetic, lane 2 i + p on part p
+// (real, imaginary) of row i: what bounds it is the number of FP64 instructions one after the other
+// (see block_sum), 2 per earlier rotation here against 12 with a thread doing them all, and one reciprocal
+// square root for the three values that need one.
 // hist (optional): the quasi-residual history, hist[nhst] written after each step.
 // lazy: the next basis vector is kept as w itself with scale 1 / ||w||.
 __device__ void givens_step(FgState *st, const double *part, int nparts, int j, int m, double tol, double *hist,
                             int lazy)
 {
-    __shared__ cplx<double> ssn[kMaxM], sc[kMaxM + 1];
-    __shared__ double scs[kMaxM];
-    if (threadIdx.x < j) {
-        scs[threadIdx.x] = st->cs[threadIdx.x];
-        ssn[threadIdx.x] = st->sn[threadIdx.x];
+    static_assert(kMaxM == 16, "one warp: two lanes per row of the column");
+    constexpr unsigned kAll = 0xffffffffu;
+    const int row = (threadIdx.x & 31) >> 1, p = threadIdx.x & 1;
+    double d = 0.0, cs = 0.0, sr = 0.0, si = 0.0, gp = 0.0, go = 0.0, gres = 0.0, rnormr0 = 0.0;
+    int nhst = 0, it = 0;
+    if (threadIdx.x < 32) {
+        if (row <= j) d = __ldcg(reinterpret_cast<const double *>(st->h) + threadIdx.x);  // CTA 0 of this launch wrote it
+        if (row < j) {
+            cs = st->cs[row];
+            sr = st->sn[row].re;
+            si = st->sn[row].im;
+        }
+        const double *g = reinterpret_cast<const double *>(st->g + j);
+        gp = g[p];
+        go = g[p ^ 1];
+        gres = st->gres;
+        rnormr0 = st->rnormr0;
+        nhst = st->hd.nhst;
+        it = st->hd.it;
     }
-    if (threadIdx.x <= j) {
-        // written by CTA 0 of the same launch: read through L2
-        const double2 v = __ldcg(reinterpret_cast<const double2 *>(st->h + threadIdx.x));
-        sc[threadIdx.x] = mk<double>(v.x, v.y);
-    }
-    const cplx<double> gj = st->g[j];
-    const double gres = st->gres, rnormr0 = st->rnormr0;
-    const int nhst = st->hd.nhst, it = st->hd.it;
     const double w2 = sum_parts_cg(part, nparts);  // ||w||^2 (synchronises the block)
-    if (threadIdx.x != 0) return;
-    FgHead &h = st->hd;
-    const double rhn = w2 > 0.0 ? rsqrt(w2) : 0.0;
-    const double hn = w2 * rhn;
-    cplx<double> *c = sc;
-    // rotations 0..j-1 on the column (c[i + 1] is the unrotated h[i + 1] for i + 1 <= j)
+    if (threadIdx.x >= 32) return;
+    const double sg = p ? 1.0 : -1.0;
+    // rotations 0..j-1 on the column: row i + 1 becomes cs d_(i+1) - conj(sn) c_i, row i cs c_i + sn d_(i+1)
+    const double dn = __shfl_down_sync(kAll, d, 2), dno = __shfl_xor_sync(kAll, dn, 1);
+    const double pn = cs * dn, ssi = sg * si;
+    double c = __shfl_sync(kAll, d, p), mine = c;
     for (int i = 0; i < j; ++i) {
-        const double ci = scs[i];
-        const cplx<double> si = ssn[i];
-        const cplx<double> t = ci * c[i] + si * c[i + 1];
-        c[i + 1] = ci * c[i + 1] - cconj(si) * c[i];
-        c[i] = t;
+        const double q = __shfl_sync(kAll, pn, 2 * i + p), ri = __shfl_sync(kAll, sr, 2 * i + p);
+        const double ii = __shfl_sync(kAll, ssi, 2 * i + p), co = __shfl_xor_sync(kAll, c, 1);
+        c = fma(ii, co, fma(-ri, c, q));
+        if (row == i + 1) mine = c;
     }
-    const cplx<double> a = c[j];
-    const double na2 = cabs2(a);
-    double cj, sabs;
-    cplx<double> sj, rjj;
+    double r = fma(ssi, dno, fma(sr, dn, cs * mine));  // row i < j
+    // the new rotation, from a = c_j and ||w||
+    const double c2 = c * c, na2 = c2 + __shfl_xor_sync(kAll, c2, 1), r2 = na2 + w2;
+    const double rs = rsqrt(row == 0 ? w2 : (row == 1 ? r2 : na2));
+    const double rw = __shfl_sync(kAll, rs, 0), rr = __shfl_sync(kAll, rs, 2), rna = __shfl_sync(kAll, rs, 4);
+    const double rhn = w2 > 0.0 ? rw : 0.0;
+    const double hn = w2 * rhn;
+    double cj, sabs, sj, rjj;
     if (w2 == 0.0) {
         cj = 1.0;
-        sj = mk<double>(0, 0);
+        sj = 0.0;
         sabs = 0.0;
-        rjj = a;
+        rjj = c;
     } else if (na2 == 0.0) {
         cj = 0.0;
-        sj = mk<double>(1.0, 0.0);
+        sj = p ? 0.0 : 1.0;
         sabs = 1.0;
-        rjj = mk<double>(hn, 0.0);
+        rjj = p ? 0.0 : hn;
     } else {
-        const double r2 = na2 + w2, rr = rsqrt(r2), rna = rsqrt(na2);
-        const cplx<double> ph = rna * a;
+        const double ph = rna * c;
         cj = na2 * rna * rr;
         sabs = hn * rr;
         sj = sabs * ph;
         rjj = (r2 * rr) * ph;
     }
-    c[j] = rjj;
+    const double so = __shfl_xor_sync(kAll, sj, 1);
+    if (row < j) reinterpret_cast<double *>(st->R + j * kMaxM)[threadIdx.x] = r;
+    if (row == j) {
+        reinterpret_cast<double *>(st->R + j * kMaxM)[threadIdx.x] = rjj;
+        reinterpret_cast<double *>(st->sn)[threadIdx.x] = sj;
+        // g(j+1) = -conj(sn) g(j), g(j) = cs g(j): the imaginary part of sn is the odd lane's
+        const double sre = p ? so : sj, sim = p ? sj : so;
+        reinterpret_cast<double *>(st->g + j + 1)[p] = fma(sg * sim, go, -(sre * gp));
+        reinterpret_cast<double *>(st->g + j)[p] = cj * gp;
+    }
+    if (threadIdx.x != 0) return;
+    FgHead &h = st->hd;
     st->cs[j] = cj;
-    st->sn[j] = sj;
-    for (int i = 0; i <= j; ++i) st->R[j * kMaxM + i] = c[i];
-    st->g[j + 1] = mk<double>(0, 0) - cconj(sj) * gj;
-    st->g[j] = cj * gj;
     const double gnew = sabs * gres;
     st->gres = gnew;
     const double q = gnew * rnormr0;
@@ -428,17 +449,17 @@ __global__ void __launch_bounds__(kThr) fg_orth_kernel(const cplx<T> *__restrict
         wout[e] = a;
         s = fma(a.re, a.re, fma(a.im, a.im, s));
     }
-    const double2 t = block_sum_t<T>(s, T(0));
+    const double t = block_sum<T>(s);
     if (!tail) {
         if (threadIdx.x == 0) {
-            part[blockIdx.x] = t.x;
+            part[blockIdx.x] = t;
             if (blockIdx.x == 0) st->pend = nv;
         }
         return;
     }
     __shared__ int last;
     if (threadIdx.x == 0) {
-        part[blockIdx.x] = t.x;
+        part[blockIdx.x] = t;
         __threadfence();
         last = atomicAdd(&st->ticket, 1) == (int)gridDim.x - 1;
     }
@@ -460,25 +481,29 @@ __global__ void __launch_bounds__(kThr) fg_finish_kernel(FgState *st, const doub
     __syncthreads();
     if (pend) givens_step(st, part, nparts, pend - 1, m, tol, hist, 1);
     __syncthreads();
-    __shared__ cplx<double> sR[kMaxM * kMaxM], sg[kMaxM], sy[kMaxM];
+    // lane 2 l + p: part p of row l; a row's diagonal enters as its reciprocal, formed for all rows at once
+    __shared__ double sR[2 * kMaxM * kMaxM];
     const int kk = st->hd.k;
-    for (int q = threadIdx.x; q < m * kMaxM; q += kThr) sR[q] = st->R[q];
-    if (threadIdx.x < m) sg[threadIdx.x] = st->g[threadIdx.x];
-    // the reciprocals of the diagonal do not wait for one another
-    __shared__ double srd[kMaxM];
+    for (int q = threadIdx.x; q < 2 * m * kMaxM; q += kThr) sR[q] = reinterpret_cast<const double *>(st->R)[q];
+    constexpr unsigned kAll = 0xffffffffu;
+    const int row = (threadIdx.x & 31) >> 1, p = threadIdx.x & 1;
+    double t = threadIdx.x < 32 && row < kk ? reinterpret_cast<const double *>(st->g)[threadIdx.x] : 0.0;
     __syncthreads();
-    if (threadIdx.x < kk) {
-        const double dd = cabs2(sR[threadIdx.x * kMaxM + threadIdx.x]);
-        srd[threadIdx.x] = dd == 0.0 ? 0.0 : 1.0 / dd;
-    }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    st->pend = 0;
+    if (threadIdx.x >= 32) return;
+    if (threadIdx.x == 0) st->pend = 0;
+    const double sg = p ? 1.0 : -1.0;
+    const double x = row < kk ? sR[2 * (row * kMaxM + row) + p] : 0.0, x2 = x * x;
+    const double dd = x2 + __shfl_xor_sync(kAll, x2, 1);
+    const double qp = -sg * x * (dd == 0.0 ? 0.0 : 1.0 / dd), qo = __shfl_xor_sync(kAll, qp, 1);
+    const double qr = p ? qo : qp, qi = sg * (p ? qp : qo);
     for (int i = kk - 1; i >= 0; --i) {
-        cplx<double> t = sg[i];
-        for (int l = i + 1; l < kk; ++l) t = t - sR[l * kMaxM + i] * sy[l];
-        sy[i] = srd[i] * (t * cconj(sR[i * kMaxM + i]));
-        st->y[i] = sy[i];
+        const double y = fma(t, qr, __shfl_xor_sync(kAll, t, 1) * qi);
+        const double yp = __shfl_sync(kAll, y, 2 * i + p), yo = __shfl_sync(kAll, y, 2 * i + (p ^ 1));
+        if (row == i) reinterpret_cast<double *>(st->y)[threadIdx.x] = y;
+        if (row < i) {
+            const double *e = sR + 2 * (i * kMaxM + row);
+            t = fma(-e[0], yp, fma(-sg * e[1], yo, t));
+        }
     }
 }
 
@@ -540,7 +565,7 @@ __device__ double sum_parts(const double *part, int nparts)
 {
     double s = 0.0;
     for (int p = threadIdx.x; p < nparts; p += kThr) s += part[p];
-    return block_sum1(s);
+    return block_sum<double>(s);
 }
 
 __device__ __forceinline__ bool cycles_left(int it, int m, long long maxit)
@@ -558,9 +583,14 @@ __global__ void __launch_bounds__(kThr) fg_norm_kernel(FgState *st, const double
 {
     fg_begin();
     if (!first && st->hd.live == 0) return;
-    const double nr = sqrt(sum_parts(part, nparts));
+    const double rnormr0 = st->rnormr0;
+    const double s = sum_parts(part, nparts);
     if (threadIdx.x != 0) return;
     FgHead &h = st->hd;
+    // one reciprocal square root in place of a root and its reciprocals
+    const bool plain = s > 0.0 && s <= DBL_MAX;
+    const double rnr = plain ? rsqrt(s) : (s != 0.0 ? 1.0 / sqrt(s) : 0.0);
+    const double nr = plain ? s * rnr : sqrt(s);
     if (first) {
         h.normr0 = nr;
         h.hst = 1.0;
@@ -571,7 +601,7 @@ __global__ void __launch_bounds__(kThr) fg_norm_kernel(FgState *st, const double
         h.live = (nr != 0.0 && h.hst > tol && cycles_left(h.it, m, maxit)) ? 1 : 0;
     } else {
         h.rn = nr;
-        if (nr / h.normr0 < tol) {
+        if (nr * rnormr0 < tol) {
             h.live = 0;
             h.conv = 1;
         } else {
@@ -580,11 +610,11 @@ __global__ void __launch_bounds__(kThr) fg_norm_kernel(FgState *st, const double
         }
     }
     h.beta = nr;
-    st->rbeta = nr != 0.0 ? 1.0 / nr : 0.0;
+    st->rbeta = rnr;
     st->gres = nr;
-    st->sv[0] = lazy ? st->rbeta : 1.0;
+    st->sv[0] = lazy ? rnr : 1.0;
     if (first) {
-        st->rnormr0 = nr != 0.0 ? 1.0 / nr : 0.0;
+        st->rnormr0 = rnr;
         st->ticket = 0;
     }
     st->pend = 0;
