@@ -42,15 +42,19 @@
 #include <cmath>
 #include <functional>
 
+#include <cooperative_groups.h>
+
 #include "h3d_kernels.cuh"
 #include "h3d_vec.cuh"
 
 namespace h3d {
+namespace cg = cooperative_groups;
 namespace {
 
 constexpr int kMaxM = 16;       // steps per cycle the state block holds
 constexpr int kMaxLevels = 8;
 constexpr int kThr = 256;
+constexpr int kCluster = 8;     // CTAs of a cluster in the inner products of the larger levels
 
 struct FgHead {                 // the part of the state the host reads
     int live;                   // the cycle loop goes on (FGMRES.m:88 and :125)
@@ -167,30 +171,46 @@ __global__ void __launch_bounds__(kThr) fg_scale_kernel(const cplx<T> *__restric
 // warp) so that kU x (vectors) independent loads are in flight before the arithmetic.
 constexpr int kU = 4;
 
+// Vectors of a kernel that goes over the basis: MV of them where the number is known at compile time
+// (kExact of them and fewer: one instance each, whose loads the compiler can all issue first), at most MV
+// otherwise.
+constexpr int kExact = 5;
+template <int MV>
+__device__ __forceinline__ int vectors(int nv)
+{
+    return MV <= kExact ? MV : nv;
+}
+
 __device__ void givens_step(FgState *st, const double *part, int nparts, int j, int m, double tol, double *hist,
                             int lazy);
 
-// Per-CTA partials of h_j = V_j^H w, j < nv <= MV: part[j * gridDim.x + cta].
+// Partials of h_j = V_j^H w, j < nv: part[j * groups + group], a group being the CTAs of a cluster (or one
+// CTA, in a launch without clusters): every CTA of the orthogonalisation adds all the partials up in FP64,
+// which at 509 partials per vector took 5 (nv = 2 or 3) to 10 us (nv = 5) of its 12 and 20, so the eight
+// CTAs of a cluster add theirs first, over distributed shared memory.
 // Stored vector 0 is u0, vector j >= 1 is V + j n (the unpreconditioned instances keep vector 0
 // in their residual buffer).
-// The last CTA (blockIdx.x = nd) runs the Givens update of the step before instead, when it is
-// outstanding: the inner products do not need it, the orthogonalisation after them does.
+// The last cluster's first CTA runs the Givens update of the step before instead, when it is
+// outstanding: the inner products do not need it, the orthogonalisation after them does.  While it is
+// outstanding the gate may close under this launch, so the gate is read only when it is not (every CTA
+// of a cluster has to take the same way).
 template <typename T, int MV>
 __global__ void __launch_bounds__(kThr) fg_dots_kernel(const cplx<T> *__restrict__ u0, const cplx<T> *__restrict__ V,
-                                                       int nv, const cplx<T> *__restrict__ w, long long n,
+                                                       int nvec, const cplx<T> *__restrict__ w, long long n,
                                                        double2 *__restrict__ part, const int *gate, FgState *st,
-                                                       const double *npart, int m, double tol, double *hist)
+                                                       const double *npart, int nparts, int m, double tol, double *hist)
 {
     fg_begin();
-    const int nd = gridDim.x - 1;
-    if ((int)blockIdx.x == nd) {
-        const int pend = st->pend;
-        if (pend == 0) return;
-        givens_step(st, npart, nd, pend - 1, m, tol, hist, 1);
-        if (threadIdx.x == 0) st->pend = 0;
+    const int nv = vectors<MV>(nvec);
+    const cg::cluster_group cl = cg::this_cluster();
+    const int gs = (int)cl.num_blocks(), nd = (int)gridDim.x - gs, ng = nd / gs;
+    const int pend = st->pend;
+    if ((int)blockIdx.x >= nd) {
+        if (pend && (int)blockIdx.x == nd) givens_step(st, npart, nparts, pend - 1, m, tol, hist, 1);
         return;
     }
-    if (closed(gate)) return;
+    if (pend == 0 && closed(gate)) return;
+    if (gs > 1) cl.barrier_arrive();  // started: its shared memory may be written
     cplx<T> acc[MV];
 #pragma unroll
     for (int j = 0; j < MV; ++j) acc[j] = mk<T>(0, 0);
@@ -242,11 +262,21 @@ __global__ void __launch_bounds__(kThr) fg_dots_kernel(const cplx<T> *__restrict
     }
     __syncthreads();
     static_assert(MV * 2 * (kThr / 32) <= kThr, "one thread per warp result");
-    if (wid * 32 >= nv * 2 * (kThr / 32)) return;  // whole warps: two vectors each
-    const int e2 = threadIdx.x, jc = e2 / (kThr / 32);
-    const double v = warps_sum8(jc < 2 * nv ? sw[e2] : 0.0);
-    if (jc < 2 * nv && (e2 & (kThr / 32 - 1)) == 0)
-        reinterpret_cast<double *>(part + (long long)(jc >> 1) * nd + blockIdx.x)[jc & 1] = v;
+    // thread 8 c + w: warp w's result of sum c (vector c / 2; real or imaginary part)
+    __shared__ double scl[kCluster * kMaxM * 2];
+    const int c = threadIdx.x / (kThr / 32);
+    const bool mine = c < 2 * nv;
+    double v = warps_sum8(mine ? sw[threadIdx.x] : 0.0);
+    const bool first = mine && (threadIdx.x & (kThr / 32 - 1)) == 0;
+    if (gs > 1) {
+        static_assert(kCluster == kThr / 32, "the leader adds a cluster's CTAs as a CTA adds its warps");
+        cl.barrier_wait();
+        if (first) cl.map_shared_rank(scl, 0)[c * kCluster + cl.block_rank()] = v;
+        cl.sync();
+        if (cl.block_rank() != 0) return;
+        v = warps_sum8(mine ? scl[threadIdx.x] : 0.0);
+    }
+    if (first) reinterpret_cast<double *>(part + (long long)(c >> 1) * ng + blockIdx.x / gs)[c & 1] = v;
 }
 
 // Sum of per-CTA partials written by other CTAs of the same launch (read through L2).
@@ -373,25 +403,51 @@ __device__ __forceinline__ void csub_mul(cplx<T> &a, cplx<T> v, cplx<T> h)
 // wout = sv[k] win - sum_j V_j h_j, k = nv - 1, with h summed here from the dots' partials (every
 // CTA in the same fixed order, so all agree; CTA 0 stores h in the state) and scaled by the
 // stored vectors' factors: the basis vector j is sv[j] times stored vector j, win = A (stored
-// vector k).  Per-CTA partials of ||wout||^2.  wout may be win.  nv <= MV.
+// vector k).  Per-CTA partials of ||wout||^2.  wout may be win, or null (a cycle's last vector, of which
+// only the norm is needed).  In complex64 the first elements are loaded before the sums, whose latency
+// they cover (6.7 us for 1-4 vectors on an 81x71x51 level without).
 // tail: the CTA that finishes last (a ticket counter in the state: every CTA publishes its partial,
 // fences, then takes a ticket; no CTA waits for another) runs the step's Givens update
 // (givens_step) for step j = nv - 1 and resets the counter.  Otherwise the update is left outstanding.
 template <typename T, int MV>
-__global__ void __launch_bounds__(kThr) fg_orth_kernel(const cplx<T> *__restrict__ u0, const cplx<T> *__restrict__ V,
-                                                       int nv, const cplx<T> *win, cplx<T> *wout, long long n,
-                                                       const double2 *__restrict__ dpart, int nparts, FgState *st,
+__global__ void __launch_bounds__(kThr, sizeof(T) == 4 && MV <= 8 ? 4 : 1) fg_orth_kernel(const cplx<T> *__restrict__ u0, const cplx<T> *__restrict__ V,
+                                                       int nvec, const cplx<T> *win, cplx<T> *wout, long long n,
+                                                       const double2 *__restrict__ dpart, int ng, FgState *st,
                                                        double *part, int m, double tol, double *hist, int tail,
                                                        const int *gate)
 {
     fg_begin();
-    if (closed(gate)) return;
+    if (closed(gate)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) st->pend = 0;
+        return;
+    }
+    const int nv = vectors<MV>(nvec);
+    // vectors whose elements are loaded ahead (registers for four CTAs per SM)
+    constexpr int kAhead = sizeof(T) == 4 && MV <= kExact ? (MV < 3 ? MV : MV < 5 ? 3 : 2) : 0;
+    const long long stride = (long long)gridDim.x * kThr;
+    long long e = blockIdx.x * (long long)kThr + threadIdx.x;
+    cplx<T> a[kU], vv[kAhead ? kAhead : 1][kU];
+    auto ahead = [&]() -> bool {
+        if (e + (kU - 1) * stride >= n) return false;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) a[u] = win[e + u * stride];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+            const cplx<T> *vj = j == 0 ? u0 : V + (long long)j * n;
+#pragma unroll
+            for (int u = 0; u < kU; ++u) vv[j][u] = vj[e + u * stride];
+        }
+        return true;
+    };
+    bool have = false;
+    if constexpr (kAhead > 0) have = ahead();
     __shared__ cplx<T> sh[kMaxM];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int j = wid; j < nv; j += kThr / 32) {
+        const double svj = st->sv[j], svk = st->sv[nv - 1];
         double re = 0.0, im = 0.0;
-        for (int p = lane; p < nparts; p += 32) {
-            const double2 v = dpart[(long long)j * nparts + p];
+        for (int p = lane; p < ng; p += 32) {
+            const double2 v = dpart[(long long)j * ng + p];
             re += v.x;
             im += v.y;
         }
@@ -404,50 +460,67 @@ __global__ void __launch_bounds__(kThr) fg_orth_kernel(const cplx<T> *__restrict
             im = __shfl_xor_sync(0xffffffffu, t, 16);
         }
         if (lane == 0) {
-            const double f = st->sv[j] * st->sv[nv - 1];
+            const double f = svj * svk;
             const cplx<double> hj = mk<double>(f * re, f * im);      // H(j+1, k+1)
-            sh[j] = mk<T>((T)(st->sv[j] * hj.re), (T)(st->sv[j] * hj.im));  // applied to stored vector j
+            sh[j] = mk<T>((T)(svj * hj.re), (T)(svj * hj.im));  // applied to stored vector j
             if (blockIdx.x == 0) st->h[j] = hj;
         }
     }
-    __syncthreads();
     const T sk = (T)st->sv[nv - 1];
+    __syncthreads();
     T s = 0;
-    const long long stride = (long long)gridDim.x * kThr;
-    long long e = blockIdx.x * (long long)kThr + threadIdx.x;
-    for (; e + (kU - 1) * stride < n; e += kU * stride) {
-        cplx<T> a[kU];
+    auto put = [&]() {
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
-            const cplx<T> t = win[e + u * stride];
-            a[u] = mk<T>(sk * t.re, sk * t.im);
+            if (wout) wout[e + u * stride] = a[u];
+            s = fma(a[u].re, a[u].re, fma(a[u].im, a[u].im, s));
         }
+    };
+    if constexpr (kAhead > 0) {
+        while (have) {
 #pragma unroll
-        for (int j = 0; j < MV; ++j) {
-            if (j < nv) {
+            for (int u = 0; u < kU; ++u) a[u] = mk<T>(sk * a[u].re, sk * a[u].im);
+#pragma unroll
+            for (int j = 0; j < MV; ++j) {
                 const cplx<T> *vj = j == 0 ? u0 : V + (long long)j * n;
-                cplx<T> v[kU];
-#pragma unroll
-                for (int u = 0; u < kU; ++u) v[u] = vj[e + u * stride];
                 const cplx<T> hj = sh[j];
 #pragma unroll
-                for (int u = 0; u < kU; ++u) csub_mul(a[u], v[u], hj);
+                for (int u = 0; u < kU; ++u) csub_mul(a[u], j < kAhead ? vv[j < kAhead ? j : 0][u] : vj[e + u * stride], hj);
             }
+            put();
+            e += kU * stride;
+            have = ahead();
         }
+    } else {
+        for (; e + (kU - 1) * stride < n; e += kU * stride) {
 #pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            wout[e + u * stride] = a[u];
-            s = fma(a[u].re, a[u].re, fma(a[u].im, a[u].im, s));
+            for (int u = 0; u < kU; ++u) {
+                const cplx<T> t = win[e + u * stride];
+                a[u] = mk<T>(sk * t.re, sk * t.im);
+            }
+#pragma unroll
+            for (int j = 0; j < MV; ++j) {
+                if (j < nv) {
+                    const cplx<T> *vj = j == 0 ? u0 : V + (long long)j * n;
+                    cplx<T> v[kU];
+#pragma unroll
+                    for (int u = 0; u < kU; ++u) v[u] = vj[e + u * stride];
+                    const cplx<T> hj = sh[j];
+#pragma unroll
+                    for (int u = 0; u < kU; ++u) csub_mul(a[u], v[u], hj);
+                }
+            }
+            put();
         }
     }
     for (; e < n; e += stride) {
         const cplx<T> t = win[e];
-        cplx<T> a = mk<T>(sk * t.re, sk * t.im);
+        cplx<T> b = mk<T>(sk * t.re, sk * t.im);
 #pragma unroll
         for (int j = 0; j < MV; ++j)
-            if (j < nv) csub_mul(a, (j == 0 ? u0 : V + (long long)j * n)[e], sh[j]);
-        wout[e] = a;
-        s = fma(a.re, a.re, fma(a.im, a.im, s));
+            if (j < nv) csub_mul(b, (j == 0 ? u0 : V + (long long)j * n)[e], sh[j]);
+        if (wout) wout[e] = b;
+        s = fma(b.re, b.re, fma(b.im, b.im, s));
     }
     const double t = block_sum<T>(s);
     if (!tail) {
@@ -490,7 +563,6 @@ __global__ void __launch_bounds__(kThr) fg_finish_kernel(FgState *st, const doub
     double t = threadIdx.x < 32 && row < kk ? reinterpret_cast<const double *>(st->g)[threadIdx.x] : 0.0;
     __syncthreads();
     if (threadIdx.x >= 32) return;
-    if (threadIdx.x == 0) st->pend = 0;
     const double sg = p ? 1.0 : -1.0;
     const double x = row < kk ? sR[2 * (row * kMaxM + row) + p] : 0.0, x2 = x * x;
     const double dd = x2 + __shfl_xor_sync(kAll, x2, 1);
@@ -509,14 +581,14 @@ __global__ void __launch_bounds__(kThr) fg_finish_kernel(FgState *st, const doub
 
 // x += sum_{j < k} B_j y_j over the steps of the cycle (FGMRES.m:117-121), y from fg_finish_kernel.
 // Stored vector 0 is u0, vector j >= 1 is B + j n; with scaled != 0 the basis vector j is sv[j]
-// times the stored one.
-template <typename T>
+// times the stored one.  MV: the steps of a full cycle where those are kExact or fewer, whose loads then
+// all go first (a cycle cut short takes the loop over its k steps), else 0.
+template <typename T, int MV>
 __global__ void __launch_bounds__(kThr) fg_xupd_kernel(cplx<T> *__restrict__ x, const cplx<T> *__restrict__ u0,
                                                        const cplx<T> *__restrict__ B, long long n, const FgState *st,
                                                        int scaled, const int *gate)
 {
     fg_begin();
-    if (closed(gate)) return;
     __shared__ cplx<T> syt[kMaxM];
     const int kk = st->hd.k;
     if (threadIdx.x < kk) {
@@ -524,24 +596,46 @@ __global__ void __launch_bounds__(kThr) fg_xupd_kernel(cplx<T> *__restrict__ x, 
         const cplx<double> yv = st->y[threadIdx.x];
         syt[threadIdx.x] = mk<T>((T)(f * yv.re), (T)(f * yv.im));
     }
+    if (closed(gate)) return;
     __syncthreads();
     const long long stride = (long long)gridDim.x * kThr;
     long long e = blockIdx.x * (long long)kThr + threadIdx.x;
-    for (; e + (kU - 1) * stride < n; e += kU * stride) {
-        cplx<T> a[kU];
+    if (MV > 0 && kk == MV) {
+        constexpr int kX = sizeof(T) == 4 ? kU : kU / 2;
+        for (; e + (kX - 1) * stride < n; e += kX * stride) {
+            cplx<T> a[kX], v[MV + 1][kX];
 #pragma unroll
-        for (int u = 0; u < kU; ++u) a[u] = mk<T>(0, 0);
-        for (int j = 0; j < kk; ++j) {
-            const cplx<T> *bj = j == 0 ? u0 : B + (long long)j * n;
-            cplx<T> v[kU];
+            for (int j = 0; j < MV; ++j)
 #pragma unroll
-            for (int u = 0; u < kU; ++u) v[u] = bj[e + u * stride];
-            const cplx<T> yj = syt[j];
+                for (int u = 0; u < kX; ++u) v[j][u] = (j == 0 ? u0 : B + (long long)j * n)[e + u * stride];
 #pragma unroll
-            for (int u = 0; u < kU; ++u) cmac(a[u], v[u], yj);
+            for (int u = 0; u < kX; ++u) a[u] = mk<T>(0, 0), v[MV][u] = x[e + u * stride];
+#pragma unroll
+            for (int j = 0; j < MV; ++j) {
+                const cplx<T> yj = syt[j];
+#pragma unroll
+                for (int u = 0; u < kX; ++u) cmac(a[u], v[j][u], yj);
+            }
+#pragma unroll
+            for (int u = 0; u < kX; ++u) x[e + u * stride] = v[MV][u] + a[u];
         }
+    } else {
+        for (; e + (kU - 1) * stride < n; e += kU * stride) {
+            cplx<T> a[kU];
 #pragma unroll
-        for (int u = 0; u < kU; ++u) x[e + u * stride] = x[e + u * stride] + a[u];
+            for (int u = 0; u < kU; ++u) a[u] = mk<T>(0, 0);
+            for (int j = 0; j < kk; ++j) {
+                const cplx<T> *bj = j == 0 ? u0 : B + (long long)j * n;
+                cplx<T> v[kU];
+#pragma unroll
+                for (int u = 0; u < kU; ++u) v[u] = bj[e + u * stride];
+                const cplx<T> yj = syt[j];
+#pragma unroll
+                for (int u = 0; u < kU; ++u) cmac(a[u], v[u], yj);
+            }
+#pragma unroll
+            for (int u = 0; u < kU; ++u) x[e + u * stride] = x[e + u * stride] + a[u];
+        }
     }
     for (; e < n; e += stride) {
         cplx<T> a = mk<T>(0, 0);
@@ -685,7 +779,7 @@ struct Fg {                     // one FGMRES instance
         Z = pre ? a.take<cplx<T>>((size_t)m * n) : nullptr;
         w = a.take<cplx<T>>(n);
         r = a.take<cplx<T>>(n);
-        dpart = a.take<double2>((size_t)kMaxM * nparts);
+        dpart = a.take<double2>((size_t)kMaxM * nparts);  // (fewer where clusters add first)
         part = a.take<double>(nparts);
         st = a.take<FgState>(1);
     }
@@ -728,17 +822,26 @@ struct Run {                    // per-call context
 // two together leave every CTA an SM of its own (the coarse levels, whose launches take a few
 // microseconds each; larger grids would crowd the SMs that free up first).
 template <typename... KA, typename... A>
-int fg_launch(Run &R, unsigned grid, void (*kern)(KA...), A... args)
+int fg_launch(Run &R, unsigned grid, unsigned cluster, void (*kern)(KA...), A... args)
 {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2]{};
+    int na = 0;
+    if (R.before > 0 && R.before + (long long)grid <= device_sms()) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = cluster;
+        attr[na].val.clusterDim.y = attr[na].val.clusterDim.z = 1;
+        ++na;
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kThr);
     cfg.stream = R.s;
-    cfg.attrs = &attr;
-    cfg.numAttrs = R.before > 0 && R.before + (long long)grid <= device_sms() ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = na;
     H3D_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...));
     R.before = grid;
     ++R.launches;
@@ -763,21 +866,24 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
     const long long n = I.n;
     const int m = I.m;
     const unsigned nb = (unsigned)I.nparts;
+    // the inner products' CTAs, in clusters where more than two per SM each have that many partials to add
+    // (287 CTAs: an FWI gradient on 81x71x51 grids 116 ms without clusters, 119 with)
+    const unsigned gs = nb > 2u * device_sms() ? kCluster : 1u, nd = (nb + gs - 1) / gs * gs;
     int rc;
     auto matvec = [&](const cplx<T> *in, cplx<T> *out) -> int {
         ++R.launches;
         return launch_mvp<T>(op, in, out, 1, R.adj, false, R.s, &R.before);
     };
     if (zero_x) {
-        H3D_FG(nb, fg_copy_kernel<T>, b, I.r, x, n, I.part);
+        H3D_FG(nb, 1u, fg_copy_kernel<T>, b, I.r, x, n, I.part);
     } else {
         if ((rc = matvec(x, I.w))) return rc;
-        H3D_FG(nb, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, nullptr);
+        H3D_FG(nb, 1u, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, nullptr);
     }
     // Unpreconditioned instances keep their basis unnormalised (each stored vector with its scale
     // in the state): no separate scaling pass per step; vector 0 is the residual buffer itself.
     const int lazy = pre ? 0 : 1;
-    H3D_FG(1u, fg_norm_kernel, I.st, I.part, I.nparts, 1, tol, m, maxit, lazy);
+    H3D_FG(1u, 1u, fg_norm_kernel, I.st, I.part, I.nparts, 1, tol, m, maxit, lazy);
     int *live = &I.st->hd.live, *go = &I.st->hd.go;
     const cplx<T> *u0 = lazy ? I.r : I.V;
     cplx<T> *basis = pre ? I.Z : I.V;
@@ -786,7 +892,7 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
             if ((rc = R.fetch(I.st))) return rc;
             if (!R.hh->live) break;
         }
-        if (!lazy) H3D_FG(nb, fg_scale_kernel<T>, I.r, I.V, n, &I.st->rbeta, live);
+        if (!lazy) H3D_FG(nb, 1u, fg_scale_kernel<T>, I.r, I.V, n, &I.st->rbeta, live);
         bool stopped = false;  // on the quasi-residual, as read by the host: no further cycle (FGMRES.m:88)
         for (int j = 0; j < m; ++j) {
             const cplx<T> *vj = j == 0 ? u0 : I.V + (long long)j * n;
@@ -803,27 +909,46 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
                 vj = zj;
             }
             if ((rc = matvec(vj, I.w))) return rc;
-            // the orthogonalised vector: straight into the next basis slot (lazy), else into w
-            cplx<T> *wout = (lazy && j + 1 < m) ? I.V + (long long)(j + 1) * n : I.w;
+            // the orthogonalised vector: straight into the next basis slot (lazy), else into w; nowhere after
+            // the last step
+            cplx<T> *wout = j + 1 == m ? nullptr : (lazy ? I.V + (long long)(j + 1) * n : I.w);
             auto step = [&](auto dots, auto orth) -> int {
-                H3D_FG(nb + 1, dots, u0, I.V, j + 1, I.w, n, I.dpart, go, I.st, I.part, m, tol, I.hist);
-                H3D_FG(nb, orth, u0, I.V, j + 1, I.w, wout, n, I.dpart, I.nparts, I.st, I.part, m, tol, I.hist,
-                       pre ? 1 : 0, go);
+                H3D_FG(nd + gs, gs, dots, u0, I.V, j + 1, I.w, n, I.dpart, go, I.st, I.part, I.nparts, m, tol, I.hist);
+                H3D_FG(nb, 1u, orth, u0, I.V, j + 1, I.w, wout, n, I.dpart, (int)(nd / gs), I.st, I.part, m, tol,
+                       I.hist, pre ? 1 : 0, go);
                 return H3D_OK;
             };
-            if (j < 4) rc = step(fg_dots_kernel<T, 4>, fg_orth_kernel<T, 4>);
-            else if (j < 8) rc = step(fg_dots_kernel<T, 8>, fg_orth_kernel<T, 8>);
-            else rc = step(fg_dots_kernel<T, kMaxM>, fg_orth_kernel<T, kMaxM>);
+            switch (j) {
+                case 0: rc = step(fg_dots_kernel<T, 1>, fg_orth_kernel<T, 1>); break;
+                case 1: rc = step(fg_dots_kernel<T, 2>, fg_orth_kernel<T, 2>); break;
+                case 2: rc = step(fg_dots_kernel<T, 3>, fg_orth_kernel<T, 3>); break;
+                case 3: rc = step(fg_dots_kernel<T, 4>, fg_orth_kernel<T, 4>); break;
+                case 4: rc = step(fg_dots_kernel<T, 5>, fg_orth_kernel<T, 5>); break;
+                case 5: case 6: case 7: rc = step(fg_dots_kernel<T, 8>, fg_orth_kernel<T, 8>); break;
+                default: rc = step(fg_dots_kernel<T, kMaxM>, fg_orth_kernel<T, kMaxM>);
+            }
             if (rc) return rc;
-            if (!lazy && j + 1 < m) H3D_FG(nb, fg_scale_kernel<T>, I.w, I.V + (long long)(j + 1) * n, n, &I.st->rhn, go);
+            if (!lazy && j + 1 < m) H3D_FG(nb, 1u, fg_scale_kernel<T>, I.w, I.V + (long long)(j + 1) * n, n, &I.st->rhn, go);
         }
-        H3D_FG(1u, fg_finish_kernel, I.st, I.part, I.nparts, m, tol, I.hist);
-        H3D_FG(nb, fg_xupd_kernel<T>, x, pre ? I.Z : u0, basis, n, I.st, lazy, live);
+        H3D_FG(1u, 1u, fg_finish_kernel, I.st, I.part, I.nparts, m, tol, I.hist);
+        auto update = [&](auto kern) -> int {
+            H3D_FG(nb, 1u, kern, x, pre ? I.Z : u0, basis, n, I.st, lazy, live);
+            return H3D_OK;
+        };
+        switch (m) {
+            case 1: rc = update(fg_xupd_kernel<T, 1>); break;
+            case 2: rc = update(fg_xupd_kernel<T, 2>); break;
+            case 3: rc = update(fg_xupd_kernel<T, 3>); break;
+            case 4: rc = update(fg_xupd_kernel<T, 4>); break;
+            case 5: rc = update(fg_xupd_kernel<T, 5>); break;
+            default: rc = update(fg_xupd_kernel<T, 0>);
+        }
+        if (rc) return rc;
         if (tail == kFgNone && (stopped || c == maxit - 1)) break;
         if ((rc = matvec(x, I.w))) return rc;
-        H3D_FG(nb, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, live);
+        H3D_FG(nb, 1u, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, live);
         if (tail == kFgResidual && c == maxit - 1) break;
-        H3D_FG(1u, fg_norm_kernel, I.st, I.part, I.nparts, 0, tol, m, maxit, lazy);
+        H3D_FG(1u, 1u, fg_norm_kernel, I.st, I.part, I.nparts, 0, tol, m, maxit, lazy);
     }
     if (tail == kFgHead) return R.fetch(I.st);
     return H3D_OK;
