@@ -1,6 +1,6 @@
 // Matrix-free matvec y = H x (and H^H x, dH x, dH^H x) as a z-marching stencil.
 //
-// A CTA owns a 32 x 8 column of rows and marches a chunk of planes in z.  Each plane of
+// A CTA owns a 32 x 4 (complex128: 32 x 8) column of rows and marches a chunk of planes in z.  Each plane of
 // x (and, forward, of the wavenumber) is staged in shared memory with its one-point xy
 // halo by asynchronous copies (double-buffered: plane p+1 streams in while plane p is
 // used).  From a plane every thread forms the partial sums of its 3 x 3 in-plane
@@ -23,9 +23,20 @@
 
 namespace h3d {
 
-constexpr int kMX = 32, kMY = 8;                 // CTA columns
-constexpr int kPX = kMX + 2, kPY = kMY + 2;      // staged plane with halo
-constexpr int kPN = kPX * kPY;
+// CTA columns: kMX x tile_rows.  What the complex64 kernel lacks is instructions to choose from (128
+// registers a thread: 16 warps per SM), and four small CTAs wait at their barriers less than two large
+// ones: 201 x 201 x 101 51.0 us with 32 x 8, 44.4 with 32 x 4 (46.2 with 32 x 2, whose halo is as large as
+// its tile); 81 x 71 x 51 10.0, 9.0 (9.2); 22 x 19 x 14 3.5, 3.1 (3.2).  More registers' worth of CTAs per SM
+// spill (five of 32 x 4: 50.0 us).  The residual kernels and complex128 keep the larger tile, and with it the
+// number of their partial sums.
+constexpr int kMX = 32;
+template <typename T, bool RESID>
+__host__ __device__ constexpr int tile_rows()
+{
+    return sizeof(T) == 4 && !RESID ? 4 : 8;
+}
+constexpr int kPX = kMX + 2;                     // row of a staged plane with its halo
+constexpr int kBufs = 3;                         // staged planes: one in use, two on their way
 
 template <int BYTES>
 __device__ __forceinline__ void mv_cp_async(void *sdst, const void *gsrc, bool valid)
@@ -47,15 +58,16 @@ __host__ __device__ inline int tile_shift(int lo, int hi, int t)
 }
 
 template <typename T, bool ADJ, bool DERIV, bool WNC, bool RESID>
-__global__ void __launch_bounds__(kMX *kMY) mvp_zmarch_kernel(Op<T> op, const cplx<T> *__restrict__ x,
+__global__ void __launch_bounds__(kMX *tile_rows<T, RESID>(), sizeof(T) == 8 ? 1 : (RESID ? 2 : 3)) mvp_zmarch_kernel(Op<T> op, const cplx<T> *__restrict__ x,
                                                               cplx<T> *__restrict__ y,
                                                               const cplx<T> *__restrict__ b, int kz,
                                                               int nchunks, double *part)
 {
+    constexpr int kMY = tile_rows<T, RESID>(), kPN = kPX * (kMY + 2);
     constexpr bool NEED_WN = !ADJ;  // forward: neighbour wavenumbers; adjoint: centre only
-    __shared__ __align__(16) cplx<T> sx[2][kPN];
-    __shared__ T swr[NEED_WN ? 2 : 1][NEED_WN ? kPN : 1];
-    __shared__ T swi[NEED_WN && WNC ? 2 : 1][NEED_WN && WNC ? kPN : 1];
+    __shared__ __align__(16) cplx<T> sx[kBufs][kPN];
+    __shared__ T swr[NEED_WN ? kBufs : 1][NEED_WN ? kPN : 1];
+    __shared__ T swi[NEED_WN && WNC ? kBufs : 1][NEED_WN && WNC ? kPN : 1];
 
     // the next launch may set up early; wait for the launch before (nothing in an ordinary launch)
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
@@ -63,8 +75,10 @@ __global__ void __launch_bounds__(kMX *kMY) mvp_zmarch_kernel(Op<T> op, const cp
     const int tid = threadIdx.x + kMX * threadIdx.y;
     const int s = blockIdx.z / nchunks, chunk = blockIdx.z % nchunks;
     const int kb = chunk * kz, ke = min(op.nz, kb + kz);
-    const int i0 = blockIdx.x * kMX - tile_shift(op.int_lo_f[0], op.int_hi_f[0], kMX);
-    const int j0 = blockIdx.y * kMY - tile_shift(op.int_lo_f[1], op.int_hi_f[1], kMY);
+    const int sx0 = tile_shift(op.int_lo_f[0], op.int_hi_f[0], kMX);
+    const unsigned gx = (unsigned)(op.nx + sx0 + kMX - 1) / kMX;  // tiles side by side in x
+    const int i0 = (int)(blockIdx.x % gx) * kMX - sx0;
+    const int j0 = (int)(blockIdx.x / gx) * kMY - tile_shift(op.int_lo_f[1], op.int_hi_f[1], kMY);
     const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
     const bool valid = i >= 0 && i < op.nx && j >= 0 && j < op.ny;
     const cplx<T> *xs = x + (long long)s * op.N;
@@ -105,7 +119,6 @@ __global__ void __launch_bounds__(kMX *kMY) mvp_zmarch_kernel(Op<T> op, const cp
                 }
             }
         }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
 
     RowPml<T> pml{};
@@ -124,15 +137,13 @@ __global__ void __launch_bounds__(kMX *kMY) mvp_zmarch_kernel(Op<T> op, const cp
     // row pk-1, whose accumulator then serves row pk+2 (its first plane sets every bracket,
     // so nothing is cleared).  The caller rotates the three accumulators' roles, so no
     // accumulator is ever copied.
-    auto step = [&](int pk, RowAcc<T> &lo, RowAcc<T> &mid, RowAcc<T> &hi) {
-        const int buf = (pk - (kb - 1)) & 1;
-        if (pk + 1 <= ke) {
-            stage(buf ^ 1, pk + 1);
-            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        }
+    // The plane after next is copied into the buffer that the barrier shows to be read to its end:
+    // one barrier a plane, and two planes of time for a copy.
+    auto step = [&](int pk, int buf, RowAcc<T> &lo, RowAcc<T> &mid, RowAcc<T> &hi) {
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();
+        if (pk + 2 <= ke) stage(buf == 0 ? 2 : buf - 1, pk + 2);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
         {
             const PlaneSums<T> P = plane_sums<T, ADJ, WNC, kPX>(sx[buf], NEED_WN ? swr[buf] : nullptr,
                                                                 NEED_WN && WNC ? swi[buf] : nullptr, l);
@@ -149,7 +160,6 @@ __global__ void __launch_bounds__(kMX *kMY) mvp_zmarch_kernel(Op<T> op, const cp
                 acc_plane<0, T, DERIV>(hi, P, op);
             }
         }
-        __syncthreads();
         const int k = pk - 1;  // row completed by this plane
         if (k >= kb && valid) {
             RowPml<T> p = pml;
@@ -188,16 +198,19 @@ __global__ void __launch_bounds__(kMX *kMY) mvp_zmarch_kernel(Op<T> op, const cp
     acc_zero(Q1);
     acc_zero(Q2);
     stage(0, kb - 1);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    stage(1, kb);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
     for (int pk = kb - 1; pk <= ke; pk += 3) {
-        step(pk, Q0, Q1, Q2);
-        if (pk + 1 <= ke) step(pk + 1, Q1, Q2, Q0);
-        if (pk + 2 <= ke) step(pk + 2, Q2, Q0, Q1);
+        step(pk, 0, Q0, Q1, Q2);
+        if (pk + 1 <= ke) step(pk + 1, 1, Q1, Q2, Q0);
+        if (pk + 2 <= ke) step(pk + 2, 2, Q2, Q0, Q1);
     }
     if constexpr (RESID) {
         const double2 t = block_sum2_r(rr, bb);
         if (tid == 0) {
-            const long long G = (long long)gridDim.x * gridDim.y * nchunks;
-            const long long blin = blockIdx.x + gridDim.x * (blockIdx.y + (long long)gridDim.y * chunk);
+            const long long G = (long long)gridDim.x * nchunks;
+            const long long blin = blockIdx.x + (long long)gridDim.x * chunk;
             part[2 * (s * G + blin)] = t.x;
             part[2 * (s * G + blin) + 1] = t.y;
         }
@@ -221,7 +234,7 @@ static int zmarch_slots()
     if (cache[dev] == 0) {
         int per_sm = 0, sms = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mvp_zmarch_kernel<T, false, false, false, RESID>,
-                                                          kMX * kMY, 0) != cudaSuccess ||
+                                                          kMX * tile_rows<T, RESID>(), 0) != cudaSuccess ||
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
             cudaGetLastError();
             per_sm = 0;
@@ -243,12 +256,13 @@ void mvp_prime_occupancy()
 // (its rows plus the two halo planes), and the launch takes as many rounds of resident CTAs
 // as the grid needs: the split minimises rounds x (chunk + 2), which balances the halo
 // overhead of short chunks against the partly empty last round of a grid that does not fill
-// the device (config 1, 201 x 201 x 101: 5 chunks of 21 planes, 910 CTAs in 3 full rounds
-// of 304).  Without an occupancy figure, chunks of 16 planes.
+// the device (201 x 201 x 101 in complex64: 5 chunks of 21 planes, 1785 CTAs in 3 rounds of
+// 608).  Without an occupancy figure, chunks of 16 planes.
 template <typename T, bool RESID>
 static dim3 zmarch_grid(const Op<T> &op, int nrhs, int *kz, int *nchunks)
 {
     const long long gx = (op.nx + tile_shift(op.int_lo_f[0], op.int_hi_f[0], kMX) + kMX - 1) / kMX;
+    constexpr int kMY = tile_rows<T, RESID>();
     const long long gy = (op.ny + tile_shift(op.int_lo_f[1], op.int_hi_f[1], kMY) + kMY - 1) / kMY;
     const int slots = zmarch_slots<T, RESID>();
     int best_kz = op.nz < 32 ? op.nz : 16;
@@ -267,7 +281,7 @@ static dim3 zmarch_grid(const Op<T> &op, int nrhs, int *kz, int *nchunks)
     }
     *kz = best_kz;
     *nchunks = (op.nz + *kz - 1) / *kz;
-    return dim3((unsigned)gx, (unsigned)gy, *nchunks * nrhs);
+    return dim3((unsigned)(gx * gy), 1, *nchunks * nrhs);  // all tiles along x: no limit on ny
 }
 
 // The flat kernel's z split: an SM works off its CTAs at a fixed rate whatever runs side by side,
@@ -388,7 +402,7 @@ static int zmarch_dispatch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const 
                   have, parts);
         return H3D_ERR_BAD_ARG;
     }
-    const dim3 blk(kMX, kMY);
+    const dim3 blk(kMX, tile_rows<T, RESID>());
     const bool wnc = op.wni != nullptr;
     int rc = H3D_OK;
     const long long ctas = (long long)grd.x * grd.y * grd.z;
