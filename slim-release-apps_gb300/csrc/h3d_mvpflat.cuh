@@ -98,10 +98,11 @@ __global__ void __launch_bounds__(kFT)
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     const int tid = threadIdx.x;
-    const int s = blockIdx.y / nchunks, chunk = blockIdx.y % nchunks;
+    const int s = blockIdx.y / nchunks, chunk = (int)outside_in(blockIdx.y % nchunks, nchunks);
+    const unsigned tile = outside_in(blockIdx.x, gridDim.x);
     const int kb = chunk * kz, ke = min(op.nz, kb + kz);
     const int nx = op.nx;
-    const long long P0 = (long long)blockIdx.x * kFT, p = P0 + tid;
+    const long long P0 = (long long)tile * kFT, p = P0 + tid;
     const bool valid = p < op.sz;
     const int j = valid ? (int)(p / nx) : 0, i = valid ? (int)(p - (long long)j * nx) : 0;
     const C *xs = x + (long long)s * op.N;
@@ -374,7 +375,7 @@ __global__ void __launch_bounds__(kFT)
         const double2 t = block_sum2_r(rr, bb);
         if (tid == 0) {
             const long long G = (long long)gridDim.x * nchunks;
-            const long long blin = blockIdx.x + (long long)gridDim.x * chunk;
+            const long long blin = tile + (long long)gridDim.x * chunk;
             part[2 * (s * G + blin)] = t.x;
             part[2 * (s * G + blin) + 1] = t.y;
         }

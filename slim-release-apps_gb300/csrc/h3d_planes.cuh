@@ -10,6 +10,12 @@
 
 namespace h3d {
 
+// Index i of n, from both ends inwards: the flat matvec hands its tiles and z chunks out this way, those
+// with PML rows (whose brackets do not fold) first and the interior last, so that the last CTAs to start
+// are short ones (161 x 161 x 81, 4 right-hand sides: 1588 us in order, 1539 so; the complex64 kernel's
+// many small CTAs gain nothing).
+__device__ __forceinline__ unsigned outside_in(unsigned i, unsigned n) { return i & 1 ? n - 1 - (i >> 1) : i >> 1; }
+
 // Plane partial sums of one thread.  W* are the mass sums: forward, weighted by the
 // neighbour's wavenumber; adjoint, unweighted (the centre wavenumber multiplies later).
 template <typename T>
