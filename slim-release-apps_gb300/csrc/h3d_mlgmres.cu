@@ -20,18 +20,18 @@
 // products V^H w (per-CTA partial sums), and the orthogonalisation w -= V h fused with the final
 // sum of those partials and with ||w||^2 partials.  The step's Givens update (the previous rotations
 // on the new Hessenberg column, the next rotation, the rotated right-hand side and the
-// quasi-residual: a dependent chain of some 100 FP64 instructions, about 5 us) runs beside the next
-// step's inner products, in a CTA of its own, or ends the cycle together with the back substitution; the
-// preconditioned instances, whose next step the host decides on, run it in the last CTA of the
-// orthogonalisation.  The basis is kept unnormalised with a scale per
+// quasi-residual: a dependent chain of FP64 instructions, about 3 us) runs beside the next step's inner
+// products, in a CTA of its own; after a cycle's last step, and in the preconditioned instances, whose next
+// step the host decides on, in the last CTA of the orthogonalisation, at the end of a cycle followed by the
+// back substitution.  The basis is kept unnormalised with a scale per
 // vector in the unpreconditioned instances; the preconditioned ones (whose basis vectors feed
 // the V-cycle) add a fourth launch, the scaling V(:,k+1) = w / ||w||.  The Givens update gives
 // the least-squares residual norm of FGMRES.m:111-113 without a host round trip; the solution y
 // is back-substituted once per cycle.  Every kernel after the matvec reads
 // a flag of the state block (the step runs / the cycle runs) and returns at once when it is
-// clear, so the host enqueues a whole unpreconditioned cycle without waiting: it
-// synchronises once per cycle there, and before each step of a preconditioned instance (to
-// decide whether the expensive preconditioner runs at all).  Sums are deterministic: fixed
+// clear, so the host enqueues unpreconditioned cycles without waiting: it synchronises once per
+// cycle of a coarse solve there, after every fourth cycle of a smoother, and before each step of
+// a preconditioned instance (to decide whether the expensive preconditioner runs at all).  Sums are deterministic: fixed
 // per-thread and per-warp sums in the field's precision, then per-CTA partials and their
 // totals in FP64 in a fixed order.
 //
@@ -131,24 +131,6 @@ __global__ void __launch_bounds__(kThr) fg_copy_kernel(const cplx<T> *__restrict
         if (x) x[e] = mk<T>(0, 0);
         s = fma(v.re, v.re, fma(v.im, v.im, s));
     }
-    const double t = block_sum<T>(s);
-    if (threadIdx.x == 0) part[blockIdx.x] = t;
-}
-
-// r = b - ax (r may alias ax); per-CTA partials of ||r||^2 when part is given.
-template <typename T>
-__global__ void __launch_bounds__(kThr) fg_sub_kernel(const cplx<T> *__restrict__ b, const cplx<T> *ax, cplx<T> *r,
-                                                      long long n, double *part, const int *gate)
-{
-    fg_begin();
-    if (closed(gate)) return;
-    T s = 0;
-    for (long long e = blockIdx.x * (long long)kThr + threadIdx.x; e < n; e += (long long)gridDim.x * kThr) {
-        const cplx<T> v = b[e] - ax[e];
-        r[e] = v;
-        s = fma(v.re, v.re, fma(v.im, v.im, s));
-    }
-    if (!part) return;
     const double t = block_sum<T>(s);
     if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
@@ -287,6 +269,103 @@ __device__ double sum_parts_cg(const double *part, int nparts)
     return block_sum<double>(s);
 }
 
+// Publish this CTA's partial t (valid in thread 0); true in the CTA of the launch that does so last.
+__device__ bool last_cta(FgState *st, double *part, double t)
+{
+    __shared__ int last;
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = t;
+        __threadfence();
+        last = atomicAdd(&st->ticket, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+__device__ __forceinline__ bool cycles_left(int it, int m, long long maxit)
+{
+    return (long long)(it / m) < maxit;  // floor(it_counter / maxinnerit) < maxit
+}
+
+// INIT (first = 1): normr0 = beta = ||r||, hst = 1, it = 1 (FGMRES.m:62-76).
+// END OF CYCLE (first = 0, while live): the true residual's norm decides the break of
+// FGMRES.m:125, then the loop condition of FGMRES.m:88.  Either way the next cycle starts
+// from beta = ||r|| (FGMRES.m:92).
+// lazy: the cycle keeps its basis unnormalised (vector 0 = r itself, scale 1 / beta).
+// Run by every thread of one CTA.
+__device__ void norm_update(FgState *st, const double *part, int nparts, int first, double tol, int m, long long maxit,
+                            int lazy)
+{
+    const double rnormr0 = st->rnormr0;
+    const double s = sum_parts_cg(part, nparts);
+    if (threadIdx.x != 0) return;
+    FgHead &h = st->hd;
+    // one reciprocal square root in place of a root and its reciprocals
+    const bool plain = s > 0.0 && s <= DBL_MAX;
+    const double rnr = plain ? rsqrt(s) : (s != 0.0 ? 1.0 / sqrt(s) : 0.0);
+    const double nr = plain ? s * rnr : sqrt(s);
+    if (first) {
+        h.normr0 = nr;
+        h.hst = 1.0;
+        h.it = 1;
+        h.nhst = 0;
+        h.conv = nr == 0.0 ? 1 : 0;
+        h.rn = nr;
+        h.live = (nr != 0.0 && h.hst > tol && cycles_left(h.it, m, maxit)) ? 1 : 0;
+    } else {
+        h.rn = nr;
+        if (nr * rnormr0 < tol) {
+            h.live = 0;
+            h.conv = 1;
+        } else {
+            if (h.hst <= tol) h.conv = 1;  // (a NaN quasi-residual stops the loop unconverged)
+            h.live = (h.hst > tol && cycles_left(h.it, m, maxit)) ? 1 : 0;
+        }
+    }
+    h.beta = nr;
+    st->rbeta = rnr;
+    st->gres = nr;
+    st->sv[0] = lazy ? rnr : 1.0;
+    if (first) st->rnormr0 = rnr;
+    st->ticket = 0;
+    st->pend = 0;
+    h.k = 0;
+    h.go = h.live;
+    st->g[0] = mk<double>(nr, 0.0);
+}
+
+__global__ void __launch_bounds__(kThr) fg_norm_kernel(FgState *st, const double *part, int nparts, double tol, int m,
+                                                       long long maxit, int lazy)
+{
+    fg_begin();
+    norm_update(st, part, nparts, 1, tol, m, maxit, lazy);
+}
+
+// r = b - ax (r may alias ax).  While the instance is live (gate) and per-CTA partials of ||r||^2 in part; with
+// st the CTA that finishes last updates the state at the end of a cycle (norm_update: the launch that
+// would do it took 3.5 us on every level).
+template <typename T>
+__global__ void __launch_bounds__(kThr) fg_sub_kernel(const cplx<T> *__restrict__ b, const cplx<T> *ax, cplx<T> *r,
+                                                      long long n, double *part, const int *gate, FgState *st,
+                                                      double tol, int m, long long maxit, int lazy)
+{
+    fg_begin();
+    if (closed(gate)) return;
+    T s = 0;
+    for (long long e = blockIdx.x * (long long)kThr + threadIdx.x; e < n; e += (long long)gridDim.x * kThr) {
+        const cplx<T> v = b[e] - ax[e];
+        r[e] = v;
+        s = fma(v.re, v.re, fma(v.im, v.im, s));
+    }
+    const double t = block_sum<T>(s);
+    if (!st) {
+        if (threadIdx.x == 0) part[blockIdx.x] = t;
+        return;
+    }
+    if (last_cta(st, part, t)) norm_update(st, part, gridDim.x, 0, tol, m, maxit, lazy);
+}
+
 // Step j of the cycle (0-based): H(1:j+1, j+1) = h, H(j+2, j+1) = ||w||; Givens rotations
 // replace the least-squares solve of FGMRES.m:111 (same solution and residual norm; y itself
 // is back-substituted once per cycle, by fg_xupd_kernel).  With H(j+2, j+1) = ||w|| real the
@@ -295,7 +374,7 @@ __device__ double sum_parts_cg(const double *part, int nparts)
 // ||w||^2), and the quasi-residual |g(j+2)| = |s| |g(j+1)| follows without a square root.
 // Run by every thread of one CTA: the one that finishes the orthogonalisation last (preconditioned
 // instances, whose next step the host decides on), an extra one of the next step's inner products, or
-// the one that ends the cycle (fg_finish_kernel).  One warp does the arithmetic, lane 2 i + p on part p
+// the one that finishes a cycle's last orthogonalisation.  One warp does the arithmetic, lane 2 i + p on part p
 // (real, imaginary) of row i: what bounds it is the number of FP64 instructions one after the other
 // (see block_sum), 2 per earlier rotation here against 12 with a thread doing them all, and one reciprocal
 // square root for the three values that need one.
@@ -390,6 +469,35 @@ __device__ void givens_step(FgState *st, const double *part, int nparts, int j, 
     h.go = (q > tol && j + 1 < m) ? 1 : 0;
 }
 
+// y = R \ g, the least-squares solution of FGMRES.m:111 after the last step, back-substituted from the
+// rotated Hessenberg matrix.  Run by every thread of one CTA.
+__device__ void back_substitute(FgState *st, int m)
+{
+    // lane 2 l + p: part p of row l; a row's diagonal enters as its reciprocal, formed for all rows at once
+    __shared__ double sR[2 * kMaxM * kMaxM];
+    const int kk = st->hd.k;
+    for (int q = threadIdx.x; q < 2 * m * kMaxM; q += kThr) sR[q] = reinterpret_cast<const double *>(st->R)[q];
+    constexpr unsigned kAll = 0xffffffffu;
+    const int row = (threadIdx.x & 31) >> 1, p = threadIdx.x & 1;
+    double t = threadIdx.x < 32 && row < kk ? reinterpret_cast<const double *>(st->g)[threadIdx.x] : 0.0;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const double sg = p ? 1.0 : -1.0;
+    const double x = row < kk ? sR[2 * (row * kMaxM + row) + p] : 0.0, x2 = x * x;
+    const double dd = x2 + __shfl_xor_sync(kAll, x2, 1);
+    const double qp = -sg * x * (dd == 0.0 ? 0.0 : 1.0 / dd), qo = __shfl_xor_sync(kAll, qp, 1);
+    const double qr = p ? qo : qp, qi = sg * (p ? qp : qo);
+    for (int i = kk - 1; i >= 0; --i) {
+        const double y = fma(t, qr, __shfl_xor_sync(kAll, t, 1) * qi);
+        const double yp = __shfl_sync(kAll, y, 2 * i + p), yo = __shfl_sync(kAll, y, 2 * i + (p ^ 1));
+        if (row == i) reinterpret_cast<double *>(st->y)[threadIdx.x] = y;
+        if (row < i) {
+            const double *e = sR + 2 * (i * kMaxM + row);
+            t = fma(-e[0], yp, fma(-sg * e[1], yo, t));
+        }
+    }
+}
+
 // a -= v * h
 template <typename T>
 __device__ __forceinline__ void csub_mul(cplx<T> &a, cplx<T> v, cplx<T> h)
@@ -406,9 +514,12 @@ __device__ __forceinline__ void csub_mul(cplx<T> &a, cplx<T> v, cplx<T> h)
 // vector k).  Per-CTA partials of ||wout||^2.  wout may be win, or null (a cycle's last vector, of which
 // only the norm is needed).  In complex64 the first elements are loaded before the sums, whose latency
 // they cover (6.7 us for 1-4 vectors on an 81x71x51 level without).
-// tail: the CTA that finishes last (a ticket counter in the state: every CTA publishes its partial,
-// fences, then takes a ticket; no CTA waits for another) runs the step's Givens update
-// (givens_step) for step j = nv - 1 and resets the counter.  Otherwise the update is left outstanding.
+// tail: with kTailStep and kTailCycle the CTA that finishes last (a ticket counter in the state: every CTA
+// publishes its partial, fences, then takes a ticket; no CTA waits for another) runs the step's Givens
+// update (givens_step) for step j = nv - 1, and with kTailCycle the back substitution that ends a cycle (as
+// CTA 0 does when the cycle's steps have stopped before), and resets the counter.  With kTailNone the
+// update is left outstanding.
+enum FgStepTail { kTailNone, kTailStep, kTailCycle };
 template <typename T, int MV>
 __global__ void __launch_bounds__(kThr, sizeof(T) == 4 && MV <= 8 ? 4 : 1) fg_orth_kernel(const cplx<T> *__restrict__ u0, const cplx<T> *__restrict__ V,
                                                        int nvec, const cplx<T> *win, cplx<T> *wout, long long n,
@@ -418,7 +529,10 @@ __global__ void __launch_bounds__(kThr, sizeof(T) == 4 && MV <= 8 ? 4 : 1) fg_or
 {
     fg_begin();
     if (closed(gate)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) st->pend = 0;
+        if (blockIdx.x == 0) {
+            if (threadIdx.x == 0) st->pend = 0;
+            if (tail == kTailCycle && st->hd.live) back_substitute(st, m);
+        }
         return;
     }
     const int nv = vectors<MV>(nvec);
@@ -523,63 +637,33 @@ __global__ void __launch_bounds__(kThr, sizeof(T) == 4 && MV <= 8 ? 4 : 1) fg_or
         s = fma(b.re, b.re, fma(b.im, b.im, s));
     }
     const double t = block_sum<T>(s);
-    if (!tail) {
+    if (tail == kTailNone) {
         if (threadIdx.x == 0) {
             part[blockIdx.x] = t;
             if (blockIdx.x == 0) st->pend = nv;
         }
         return;
     }
-    __shared__ int last;
+    if (!last_cta(st, part, t)) return;
+    givens_step(st, part, gridDim.x, nv - 1, m, tol, hist, tail == kTailCycle ? 1 : 0);
     if (threadIdx.x == 0) {
-        part[blockIdx.x] = t;
-        __threadfence();
-        last = atomicAdd(&st->ticket, 1) == (int)gridDim.x - 1;
+        st->ticket = 0;
+        st->pend = 0;
     }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    givens_step(st, part, gridDim.x, nv - 1, m, tol, hist, 0);
-    if (threadIdx.x == 0) st->ticket = 0;
+    if (tail == kTailCycle) {
+        __syncthreads();
+        back_substitute(st, m);
+    }
 }
 
-// End of a cycle's steps, one CTA: the outstanding Givens update, then y = R \ g, the least-squares
-// solution of FGMRES.m:111 after the last step, back-substituted from the rotated Hessenberg matrix.
-__global__ void __launch_bounds__(kThr) fg_finish_kernel(FgState *st, const double *part, int nparts, int m, double tol,
-                                                         double *hist)
+// End of a preconditioned instance's cycle, one CTA (the host may have ended it before its last step).
+__global__ void __launch_bounds__(kThr) fg_finish_kernel(FgState *st, int m)
 {
     fg_begin();
-    if (st->hd.live == 0) return;
-    const int pend = st->pend;
-    __syncthreads();
-    if (pend) givens_step(st, part, nparts, pend - 1, m, tol, hist, 1);
-    __syncthreads();
-    // lane 2 l + p: part p of row l; a row's diagonal enters as its reciprocal, formed for all rows at once
-    __shared__ double sR[2 * kMaxM * kMaxM];
-    const int kk = st->hd.k;
-    for (int q = threadIdx.x; q < 2 * m * kMaxM; q += kThr) sR[q] = reinterpret_cast<const double *>(st->R)[q];
-    constexpr unsigned kAll = 0xffffffffu;
-    const int row = (threadIdx.x & 31) >> 1, p = threadIdx.x & 1;
-    double t = threadIdx.x < 32 && row < kk ? reinterpret_cast<const double *>(st->g)[threadIdx.x] : 0.0;
-    __syncthreads();
-    if (threadIdx.x >= 32) return;
-    const double sg = p ? 1.0 : -1.0;
-    const double x = row < kk ? sR[2 * (row * kMaxM + row) + p] : 0.0, x2 = x * x;
-    const double dd = x2 + __shfl_xor_sync(kAll, x2, 1);
-    const double qp = -sg * x * (dd == 0.0 ? 0.0 : 1.0 / dd), qo = __shfl_xor_sync(kAll, qp, 1);
-    const double qr = p ? qo : qp, qi = sg * (p ? qp : qo);
-    for (int i = kk - 1; i >= 0; --i) {
-        const double y = fma(t, qr, __shfl_xor_sync(kAll, t, 1) * qi);
-        const double yp = __shfl_sync(kAll, y, 2 * i + p), yo = __shfl_sync(kAll, y, 2 * i + (p ^ 1));
-        if (row == i) reinterpret_cast<double *>(st->y)[threadIdx.x] = y;
-        if (row < i) {
-            const double *e = sR + 2 * (i * kMaxM + row);
-            t = fma(-e[0], yp, fma(-sg * e[1], yo, t));
-        }
-    }
+    if (st->hd.live) back_substitute(st, m);
 }
 
-// x += sum_{j < k} B_j y_j over the steps of the cycle (FGMRES.m:117-121), y from fg_finish_kernel.
+// x += sum_{j < k} B_j y_j over the steps of the cycle (FGMRES.m:117-121), y from back_substitute.
 // Stored vector 0 is u0, vector j >= 1 is B + j n; with scaled != 0 the basis vector j is sv[j]
 // times the stored one.  MV: the steps of a full cycle where those are kExact or fewer, whose loads then
 // all go first (a cycle cut short takes the loop over its k steps), else 0.
@@ -651,70 +735,6 @@ __global__ void __launch_bounds__(kThr) fg_cast_kernel(const cplx<S> *__restrict
 {
     for (long long e = blockIdx.x * (long long)kThr + threadIdx.x; e < n; e += (long long)gridDim.x * kThr)
         b[e] = mk<D>((D)a[e].re, (D)a[e].im);
-}
-
-// ---- single-CTA state updates ---------------------------------------------------------------
-
-__device__ double sum_parts(const double *part, int nparts)
-{
-    double s = 0.0;
-    for (int p = threadIdx.x; p < nparts; p += kThr) s += part[p];
-    return block_sum<double>(s);
-}
-
-__device__ __forceinline__ bool cycles_left(int it, int m, long long maxit)
-{
-    return (long long)(it / m) < maxit;  // floor(it_counter / maxinnerit) < maxit
-}
-
-// INIT (first = 1): normr0 = beta = ||r||, hst = 1, it = 1 (FGMRES.m:62-76).
-// END OF CYCLE (first = 0, runs while live): the true residual's norm decides the break of
-// FGMRES.m:125, then the loop condition of FGMRES.m:88.  Either way the next cycle starts
-// from beta = ||r|| (FGMRES.m:92).
-// lazy: the cycle keeps its basis unnormalised (vector 0 = r itself, scale 1 / beta).
-__global__ void __launch_bounds__(kThr) fg_norm_kernel(FgState *st, const double *part, int nparts, int first,
-                                                       double tol, int m, long long maxit, int lazy)
-{
-    fg_begin();
-    if (!first && st->hd.live == 0) return;
-    const double rnormr0 = st->rnormr0;
-    const double s = sum_parts(part, nparts);
-    if (threadIdx.x != 0) return;
-    FgHead &h = st->hd;
-    // one reciprocal square root in place of a root and its reciprocals
-    const bool plain = s > 0.0 && s <= DBL_MAX;
-    const double rnr = plain ? rsqrt(s) : (s != 0.0 ? 1.0 / sqrt(s) : 0.0);
-    const double nr = plain ? s * rnr : sqrt(s);
-    if (first) {
-        h.normr0 = nr;
-        h.hst = 1.0;
-        h.it = 1;
-        h.nhst = 0;
-        h.conv = nr == 0.0 ? 1 : 0;
-        h.rn = nr;
-        h.live = (nr != 0.0 && h.hst > tol && cycles_left(h.it, m, maxit)) ? 1 : 0;
-    } else {
-        h.rn = nr;
-        if (nr * rnormr0 < tol) {
-            h.live = 0;
-            h.conv = 1;
-        } else {
-            if (h.hst <= tol) h.conv = 1;  // (a NaN quasi-residual stops the loop unconverged)
-            h.live = (h.hst > tol && cycles_left(h.it, m, maxit)) ? 1 : 0;
-        }
-    }
-    h.beta = nr;
-    st->rbeta = rnr;
-    st->gres = nr;
-    st->sv[0] = lazy ? rnr : 1.0;
-    if (first) {
-        st->rnormr0 = rnr;
-        st->ticket = 0;
-    }
-    st->pend = 0;
-    h.k = 0;
-    h.go = h.live;
-    st->g[0] = mk<double>(nr, 0.0);
 }
 
 // ---- host side -------------------------------------------------------------------------------
@@ -874,16 +894,16 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
         ++R.launches;
         return launch_mvp<T>(op, in, out, 1, R.adj, false, R.s, &R.before);
     };
+    // Unpreconditioned instances keep their basis unnormalised (each stored vector with its scale
+    // in the state): no separate scaling pass per step; vector 0 is the residual buffer itself.
+    const int lazy = pre ? 0 : 1;
     if (zero_x) {
         H3D_FG(nb, 1u, fg_copy_kernel<T>, b, I.r, x, n, I.part);
     } else {
         if ((rc = matvec(x, I.w))) return rc;
-        H3D_FG(nb, 1u, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, nullptr);
+        H3D_FG(nb, 1u, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, nullptr, nullptr, tol, m, maxit, lazy);
     }
-    // Unpreconditioned instances keep their basis unnormalised (each stored vector with its scale
-    // in the state): no separate scaling pass per step; vector 0 is the residual buffer itself.
-    const int lazy = pre ? 0 : 1;
-    H3D_FG(1u, 1u, fg_norm_kernel, I.st, I.part, I.nparts, 1, tol, m, maxit, lazy);
+    H3D_FG(1u, 1u, fg_norm_kernel, I.st, I.part, I.nparts, tol, m, maxit, lazy);
     int *live = &I.st->hd.live, *go = &I.st->hd.go;
     const cplx<T> *u0 = lazy ? I.r : I.V;
     cplx<T> *basis = pre ? I.Z : I.V;
@@ -915,7 +935,7 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
             auto step = [&](auto dots, auto orth) -> int {
                 H3D_FG(nd + gs, gs, dots, u0, I.V, j + 1, I.w, n, I.dpart, go, I.st, I.part, I.nparts, m, tol, I.hist);
                 H3D_FG(nb, 1u, orth, u0, I.V, j + 1, I.w, wout, n, I.dpart, (int)(nd / gs), I.st, I.part, m, tol,
-                       I.hist, pre ? 1 : 0, go);
+                       I.hist, pre ? kTailStep : j + 1 == m ? kTailCycle : kTailNone, go);
                 return H3D_OK;
             };
             switch (j) {
@@ -930,7 +950,7 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
             if (rc) return rc;
             if (!lazy && j + 1 < m) H3D_FG(nb, 1u, fg_scale_kernel<T>, I.w, I.V + (long long)(j + 1) * n, n, &I.st->rhn, go);
         }
-        H3D_FG(1u, 1u, fg_finish_kernel, I.st, I.part, I.nparts, m, tol, I.hist);
+        if (pre) H3D_FG(1u, 1u, fg_finish_kernel, I.st, m);
         auto update = [&](auto kern) -> int {
             H3D_FG(nb, 1u, kern, x, pre ? I.Z : u0, basis, n, I.st, lazy, live);
             return H3D_OK;
@@ -946,9 +966,8 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
         if (rc) return rc;
         if (tail == kFgNone && (stopped || c == maxit - 1)) break;
         if ((rc = matvec(x, I.w))) return rc;
-        H3D_FG(nb, 1u, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, live);
-        if (tail == kFgResidual && c == maxit - 1) break;
-        H3D_FG(1u, 1u, fg_norm_kernel, I.st, I.part, I.nparts, 0, tol, m, maxit, lazy);
+        const bool end = tail == kFgResidual && c == maxit - 1;
+        H3D_FG(nb, 1u, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, live, end ? nullptr : I.st, tol, m, maxit, lazy);
     }
     if (tail == kFgHead) return R.fetch(I.st);
     return H3D_OK;
