@@ -1,7 +1,7 @@
 // Batched BLOCK8 Kaczmarz double sweep over a table of problems (h3d_b8batch.cu; the complex64
 // kernel in h3d_b8slab.cu).
 //
-// One launch per block parity covers every (problem, block, group of R right-hand sides) of
+// One launch per block parity (complex128: or one in all, see h3d_b8batch.cu) covers every (problem, block, group of R right-hand sides) of
 // the batch: problems may differ in grid size, PML, wavenumber (frequency) and mode, and each
 // keeps its own stored row coefficients.  A CTA finds its problem by a binary search over the
 // per-parity prefix counts of CTAs, copies the problem's descriptor into shared memory, and
@@ -33,6 +33,7 @@ struct B8Prob {
     int adj;              // 1: rows of H^H
     int wnc;              // complex wavenumber (no real-coefficient interior blocks)
     int NI, NJ, NK;       // 12^3 blocks per axis
+    int done0;            // complex128: index of its first (block, group) in the sweep's progress counters
 };
 
 // Compiled (precision, R, S) configurations of the batched kernel.
@@ -55,6 +56,8 @@ struct B8Batch {
     std::vector<Item> items;
     std::vector<std::unique_ptr<DevBuf>> coefs, rinvs;
     DevBuf desc, starts, errb;
+    DevBuf flow;                              // complex128: ticket counter and progress counters (see the kernel)
+    long long nflow = 0;                      // progress counters
     B8Prob<T> first;                          // host copy of the first problem's descriptor
     int cfg = -1;
     long long nctas[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -79,6 +82,8 @@ struct B8Batch {
     // One forward + backward sweep on x (all columns of the batch) with right-hand side b
     // (null = 0); active: per-column flags (null = all); selftest: see the kernel.
     int dsweep(cplx<T> *x, const cplx<T> *b, T w, const int *active, cudaStream_t st, int selftest = 0);
+    // Whether a double sweep is one launch that hands the blocks out (see the kernel).
+    bool in_one_launch() const;
     // Kernel launches of one double sweep (parities without blocks are skipped).
     int launches() const;
     // Time every configuration whose groups the columns fill on the scratch vector y (its
