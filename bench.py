@@ -76,9 +76,9 @@ REF_ITERS_CONFIG1 = 1481
 # Row order of the timed solves (the solver's tuner then picks the kernel configuration).
 DEFAULT_ORDER = "block8"
 
-# DRAM bytes (read + write) per launch of the dominant kernel from one ncu capture of the
-# complex64 config-1 solve, keyed by (order, tuned variant).
-TRAFFIC_PER_LAUNCH = {("block8", 0): 112.6e6}
+# DRAM bytes (read + write) per launch of the dominant kernel from one ncu capture of a complex64
+# sweep of the config-1 grid (cold cache), keyed by (order, tuned variant).
+TRAFFIC_PER_LAUNCH = {("block8", 0): 26.6e6}
 
 
 def _peaks():
@@ -306,7 +306,7 @@ def run_reference_arm(args, world, rank):
 
 
 # ---- the GPU arm ----------------------------------------------------------------------------------
-KERNEL = "sweep_b8_kernel<float> (batched BLOCK8 parity phase)"
+KERNEL = "sweep_slab_kernel (complex64 BLOCK8 parity phase)"
 
 
 def run_batched(args):
@@ -521,7 +521,7 @@ def run_gpu_arm(args, world, rank):
     sb = sum(i["sweep_bytes"] for i in infos)
     ss = sum(i["sweep_seconds"] for i in infos)
     sn = sum(i["sweep_samples"] for i in infos)
-    roof = _roofline(sb, ss, sn, 15, "sweep_b8_kernel<float, 1, 3> (BLOCK8 parity phase, one right-hand side)",
+    roof = _roofline(sb, ss, sn, 15, "sweep_slab_kernel<1> (complex64 BLOCK8 parity phase, one right-hand side)",
                      args.traffic_per_launch if args.traffic_per_launch is not None
                      else TRAFFIC_PER_LAUNCH.get((args.order, infos[-1]["sweep_variant"])))
     cpu = None

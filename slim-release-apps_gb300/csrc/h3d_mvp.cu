@@ -336,9 +336,9 @@ static dim3 flat_grid(const Op<T> &op, int nrhs, int *kz, int *nchunks)
 }
 
 // Whether the flat kernel takes a grid: complex128 (bound by the FP64 unit), and staged planes (one
-// row more on either side of 256 points) that leave room for two CTAs per SM.  In complex64 the
-// column tiles are faster (201 x 201 x 101: 53 us against 89): what counts there is instructions, and
-// a row more on either side of 256 points is three times the copies of a 34 x 10 tile.
+// row more on either side of 128 points) that leave room for two CTAs per SM.  In complex64 the
+// column tiles are faster (201 x 201 x 101: 44 us against 89): what counts there is instructions, and
+// a row more on either side of 128 points is many times the copies of a 34 x 6 tile.
 template <typename T>
 static bool use_flat(const Op<T> &op)
 {
