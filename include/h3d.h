@@ -216,8 +216,8 @@ int h3d_residual_noalloc(const h3d_grid *g, const double *wn_re, const double *w
                          int nrhs, int mode, void *stream);
 
 /* ---- diagnostics ------------------------------------------------------------------------ */
-/* Checks the bounded waits of the BLOCK8 sweep kernel on this GPU (no counterpart in the
- * reference).  Runs one double sweep on an internal 24^3 problem in which the kernel's first
+/* Checks the bounded waits of the complex128 BLOCK8 sweep kernel on this GPU (no counterpart in the
+ * reference).  Runs one double sweep on an internal 24^3 complex128 problem in which the kernel's first
  * colour step announces a coefficient copy on its mbarrier but never issues it, with every
  * wait limited to limit_ms (0 < limit_ms <= 1000): each CTA gives up after the limit, records
  * the expired wait in the sweep's status word and returns.  Returns H3D_ERR_TIMEOUT when that
