@@ -203,9 +203,9 @@ int h3d_residual(const h3d_grid *g, const double *wn_re, const double *wn_im, co
  * All scratch (the PML tables and the per-block partial sums) lives in one fixed device
  * array of H3D_NOALLOC_SCRATCH_BYTES that every GPU loading the library holds until the
  * process exits; grids and nrhs needing more are rejected with H3D_ERR_BAD_ARG, before any
- * launch.  The scratch holds one partial sum per 32x8-column block, z chunk and right-hand
- * side, and the z split follows the current device's occupancy, so the largest problem
- * accepted depends on the device.  The
+ * launch.  The scratch holds one partial sum per tile of a z plane (128 points, or 32x8
+ * columns where sums by the former would not fit), z chunk and right-hand side, and the z
+ * split follows the current device, so the largest problem accepted depends on it.  The
  * first call on a device looks up that array's address (once per device, with the device
  * current); make the first call before any stream capture.  Every call reuses the same
  * array, so calls that overlap on the GPU (other streams, other threads) race: serialise

@@ -25,7 +25,10 @@ __device__ __forceinline__ cplx<float> load_cg(const cplx<float> *p)
 // mvp_prime_occupancy: fixes the device occupancy the matvec grids are cut by (called when
 // an operator is made).
 void mvp_prime_occupancy();
-int mvp_residual_parts(const Op<double> &op, int nrhs);
+// Partial sums of the residual per right-hand side; most: what the caller's buffer holds of them for all
+// right-hand sides (-1: any number).  The count is that of the kernel that will run: the flat one, or where
+// its count is above most the tiled one, which the count alone then selects in launch_residual.
+int mvp_residual_parts(const Op<double> &op, int nrhs, long long most = -1);
 // parts: the partial-sum count per right-hand side the buffer was sized for
 // (mvp_residual_parts); a launch needing another count is refused.
 int launch_residual(const Op<double> &op, const cplx<double> *b, const cplx<double> *x, cplx<double> *r,

@@ -306,8 +306,9 @@ static int device_sms()
     return cache[dev];
 }
 
-// RESID: at most the partial sums per right-hand side of the tiled kernel's grid, so that what fits a
-// fixed partial-sum buffer with that kernel fits it with this one.
+// RESID: a split in z takes at most the partial sums per right-hand side of the tiled kernel's grid. One
+// chunk may take more (a tile is 128 points here, 256 there): mvp_residual_parts turns to the tiled kernel
+// where a caller's buffer is too small for that.
 template <typename T, bool RESID>
 static dim3 flat_grid(const Op<T> &op, int nrhs, int *kz, int *nchunks)
 {
@@ -389,8 +390,13 @@ static int zmarch_dispatch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const 
         return H3D_ERR_NSIZE;
     }
     int kz, nch;
-    const bool flat = use_flat(op);
-    const dim3 grd = flat ? flat_grid<T, RESID>(op, nrhs, &kz, &nch) : zmarch_grid<T, RESID>(op, nrhs, &kz, &nch);
+    bool flat = use_flat(op);
+    dim3 grd;
+    if (flat) {
+        grd = flat_grid<T, RESID>(op, nrhs, &kz, &nch);
+        if (RESID && (long long)grd.x * nch != parts) flat = false;  // sized for the tiled kernel
+    }
+    if (!flat) grd = zmarch_grid<T, RESID>(op, nrhs, &kz, &nch);
     if ((long long)nch * nrhs > 65535) {
         set_error("too many right-hand sides for one launch");
         return H3D_ERR_BAD_ARG;
@@ -434,12 +440,12 @@ int launch_mvp(const Op<T> &op, const cplx<T> *x, cplx<T> *y, int nrhs, bool adj
     return zmarch_dispatch<T, false>(op, x, y, nullptr, nrhs, adj, deriv, nullptr, 0, st, before);
 }
 
-int mvp_residual_parts(const Op<double> &op, int nrhs)
+int mvp_residual_parts(const Op<double> &op, int nrhs, long long most)
 {
     int kz, nch;
     if (use_flat(op)) {
         const dim3 g = flat_grid<double, true>(op, nrhs, &kz, &nch);
-        return (int)(g.x * nch);
+        if (most < 0 || (long long)g.x * nch * nrhs <= most) return (int)(g.x * nch);
     }
     const dim3 g = zmarch_grid<double, true>(op, nrhs, &kz, &nch);
     return (int)(g.x * g.y * nch);

@@ -73,7 +73,8 @@ extern "C" int h3d_residual_noalloc(const h3d_grid *g, const double *wn_re, cons
     probe.nx = g->n[0];
     probe.ny = g->n[1];
     probe.nz = g->n[2];
-    const long long G = mvp_residual_parts(probe, nrhs);
+    const long long room = ((long long)kNoAllocDoubles - (long long)tab_doubles) / 2;  // partial sums
+    const long long G = mvp_residual_parts(probe, nrhs, room > 0 ? room : 0);
     const size_t need = tab_doubles + 2 * (size_t)G * (size_t)nrhs;
     if (need > kNoAllocDoubles) {
         set_error("h3d_residual_noalloc: grid %dx%dx%d with %d right-hand sides needs %zu bytes of scratch, "
