@@ -36,10 +36,10 @@ int launch_residual(const Op<double> &op, const cplx<double> *b, const cplx<doub
 
 // h3d_mvp.cu / h3d_stencil.cu
 // before (optional): CTAs of the launch before on the stream if that launch lets this one set up early
-// (-1: it does not); set to this launch's CTAs.
+// (-1: it does not); set to this launch's CTAs.  gate (optional): device flag, 0: y is left as it is.
 template <typename T>
 int launch_mvp(const Op<T> &op, const cplx<T> *x, cplx<T> *y, int nrhs, bool adj, bool deriv,
-               cudaStream_t st, long long *before = nullptr);
+               cudaStream_t st, long long *before = nullptr, const int *gate = nullptr);
 // rinv: optional 1/||a_i||^2 per row (COLOUR27 only; NULL = computed in the kernel);
 // shape: COLOUR27 tile shape index (-1 = chosen from the grid).  coef (with rinv): stored
 // row coefficients; COLOUR27 then runs the direct kernel instead of the tile kernel.

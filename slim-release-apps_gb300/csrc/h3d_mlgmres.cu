@@ -890,9 +890,11 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
     // (287 CTAs: an FWI gradient on 81x71x51 grids 116 ms without clusters, 119 with)
     const unsigned gs = nb > 2u * device_sms() ? kCluster : 1u, nd = (nb + gs - 1) / gs * gs;
     int rc;
-    auto matvec = [&](const cplx<T> *in, cplx<T> *out) -> int {
+    // gate: as the kernels after it have it.  A step's matvec runs before the Givens update that may stop the
+    // instance, so it sees the flag one step late: one matvec more than needed at most.
+    auto matvec = [&](const cplx<T> *in, cplx<T> *out, const int *gate) -> int {
         ++R.launches;
-        return launch_mvp<T>(op, in, out, 1, R.adj, false, R.s, &R.before);
+        return launch_mvp<T>(op, in, out, 1, R.adj, false, R.s, &R.before, gate);
     };
     // Unpreconditioned instances keep their basis unnormalised (each stored vector with its scale
     // in the state): no separate scaling pass per step; vector 0 is the residual buffer itself.
@@ -900,7 +902,7 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
     if (zero_x) {
         H3D_FG(nb, 1u, fg_copy_kernel<T>, b, I.r, x, n, I.part);
     } else {
-        if ((rc = matvec(x, I.w))) return rc;
+        if ((rc = matvec(x, I.w, nullptr))) return rc;
         H3D_FG(nb, 1u, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, nullptr, nullptr, tol, m, maxit, lazy);
     }
     H3D_FG(1u, 1u, fg_norm_kernel, I.st, I.part, I.nparts, tol, m, maxit, lazy);
@@ -928,7 +930,7 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
                 if ((rc = (*pre)(vj, zj))) return rc;
                 vj = zj;
             }
-            if ((rc = matvec(vj, I.w))) return rc;
+            if ((rc = matvec(vj, I.w, pre ? nullptr : go))) return rc;
             // the orthogonalised vector: straight into the next basis slot (lazy), else into w; nowhere after
             // the last step
             cplx<T> *wout = j + 1 == m ? nullptr : (lazy ? I.V + (long long)(j + 1) * n : I.w);
@@ -965,7 +967,7 @@ int fgmres(Run &R, Fg<T> &I, const Op<T> &op, const cplx<T> *b, cplx<T> *x, bool
         }
         if (rc) return rc;
         if (tail == kFgNone && (stopped || c == maxit - 1)) break;
-        if ((rc = matvec(x, I.w))) return rc;
+        if ((rc = matvec(x, I.w, live))) return rc;
         const bool end = tail == kFgResidual && c == maxit - 1;
         H3D_FG(nb, 1u, fg_sub_kernel<T>, b, I.w, I.r, n, I.part, live, end ? nullptr : I.st, tol, m, maxit, lazy);
     }

@@ -61,7 +61,7 @@ template <typename T, bool ADJ, bool DERIV, bool WNC, bool RESID>
 __global__ void __launch_bounds__(kMX *tile_rows<T, RESID>(), sizeof(T) == 8 ? 1 : (RESID ? 2 : 3)) mvp_zmarch_kernel(Op<T> op, const cplx<T> *__restrict__ x,
                                                               cplx<T> *__restrict__ y,
                                                               const cplx<T> *__restrict__ b, int kz,
-                                                              int nchunks, double *part)
+                                                              int nchunks, double *part, const int *gate)
 {
     constexpr int kMY = tile_rows<T, RESID>(), kPN = kPX * (kMY + 2);
     constexpr bool NEED_WN = !ADJ;  // forward: neighbour wavenumbers; adjoint: centre only
@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(kMX *tile_rows<T, RESID>(), sizeof(T) == 8 ? 1
     // the next launch may set up early; wait for the launch before (nothing in an ordinary launch)
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    if (gate && *gate == 0) return;
     const int tid = threadIdx.x + kMX * threadIdx.y;
     const int s = blockIdx.z / nchunks, chunk = blockIdx.z % nchunks;
     const int kb = chunk * kz, ke = min(op.nz, kb + kz);
@@ -366,7 +367,7 @@ static int mvp_start(void (*kern)(KA...), dim3 grd, dim3 blk, size_t smem, bool 
 
 template <typename T, bool ADJ, bool DERIV, bool WNC, bool RESID>
 static int flat_launch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const cplx<T> *b, dim3 grd, int kz, int nch,
-                       double *part, bool early, cudaStream_t st)
+                       double *part, const int *gate, bool early, cudaStream_t st)
 {
     if constexpr (sizeof(T) == 8) {
         const size_t smem = flat_smem<T, ADJ, WNC>(op.nx);
@@ -375,7 +376,7 @@ static int flat_launch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const cplx
             H3D_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         auto aligned = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
         const int vec = aligned(x) && aligned(op.wn) && (!WNC || aligned(op.wni));
-        return mvp_start(kern, grd, dim3(kFT), smem, early, st, op, x, y, b, kz, nch, vec, part);
+        return mvp_start(kern, grd, dim3(kFT), smem, early, st, op, x, y, b, kz, nch, vec, part, gate);
     }
     return H3D_OK;
 }
@@ -383,7 +384,7 @@ static int flat_launch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const cplx
 template <typename T, bool RESID>
 static int zmarch_dispatch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const cplx<T> *b, int nrhs,
                            bool adj, bool deriv, double *part, int parts, cudaStream_t st,
-                           long long *before = nullptr)
+                           long long *before = nullptr, const int *gate = nullptr)
 {
     if ((long long)op.nx * op.ny >= (1LL << 31)) {
         set_error("a z plane of more than 2^31 - 1 points is not supported by the matvec");
@@ -415,8 +416,8 @@ static int zmarch_dispatch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const 
     const bool early = before && *before > 0 && *before + ctas <= device_sms();
     if (before) *before = ctas;
 #define H3D_ZM(A, D, W)                                                                                   \
-    if (flat) rc = flat_launch<T, A, D, W, RESID>(op, x, y, b, grd, kz, nch, part, early, st);              \
-    else rc = mvp_start(mvp_zmarch_kernel<T, A, D, W, RESID>, grd, blk, 0, early, st, op, x, y, b, kz, nch, part)
+    if (flat) rc = flat_launch<T, A, D, W, RESID>(op, x, y, b, grd, kz, nch, part, gate, early, st);        \
+    else rc = mvp_start(mvp_zmarch_kernel<T, A, D, W, RESID>, grd, blk, 0, early, st, op, x, y, b, kz, nch, part, gate)
     switch ((adj ? 4 : 0) + (deriv ? 2 : 0) + (wnc ? 1 : 0)) {
     case 0: H3D_ZM(false, false, false); break;
     case 1: H3D_ZM(false, false, true); break;
@@ -435,9 +436,9 @@ static int zmarch_dispatch(const Op<T> &op, const cplx<T> *x, cplx<T> *y, const 
 
 template <typename T>
 int launch_mvp(const Op<T> &op, const cplx<T> *x, cplx<T> *y, int nrhs, bool adj, bool deriv,
-               cudaStream_t st, long long *before)
+               cudaStream_t st, long long *before, const int *gate)
 {
-    return zmarch_dispatch<T, false>(op, x, y, nullptr, nrhs, adj, deriv, nullptr, 0, st, before);
+    return zmarch_dispatch<T, false>(op, x, y, nullptr, nrhs, adj, deriv, nullptr, 0, st, before, gate);
 }
 
 int mvp_residual_parts(const Op<double> &op, int nrhs, long long most)
@@ -457,7 +458,7 @@ int launch_residual(const Op<double> &op, const cplx<double> *b, const cplx<doub
     return zmarch_dispatch<double, true>(op, x, r, b, nrhs, adj, false, part, parts, st);
 }
 
-template int launch_mvp<double>(const Op<double> &, const cplx<double> *, cplx<double> *, int, bool, bool, cudaStream_t, long long *);
-template int launch_mvp<float>(const Op<float> &, const cplx<float> *, cplx<float> *, int, bool, bool, cudaStream_t, long long *);
+template int launch_mvp<double>(const Op<double> &, const cplx<double> *, cplx<double> *, int, bool, bool, cudaStream_t, long long *, const int *);
+template int launch_mvp<float>(const Op<float> &, const cplx<float> *, cplx<float> *, int, bool, bool, cudaStream_t, long long *, const int *);
 
 }  // namespace h3d

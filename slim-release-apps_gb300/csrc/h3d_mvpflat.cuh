@@ -85,7 +85,7 @@ __device__ __forceinline__ void flat_stage(E *dst, const E *a, long long n, long
 template <typename T, bool ADJ, bool DERIV, bool WNC, bool RESID>
 __global__ void __launch_bounds__(kFT)
     mvp_flat_kernel(const __grid_constant__ Op<T> op, const cplx<T> *__restrict__ x, cplx<T> *__restrict__ y,
-                    const cplx<T> *__restrict__ b, int kz, int nchunks, int vec, double *part)
+                    const cplx<T> *__restrict__ b, int kz, int nchunks, int vec, double *part, const int *gate)
 {
     using C = cplx<T>;
     constexpr bool NEED_WN = !ADJ;   // forward: neighbour wavenumbers; adjoint: the centre's, at the end
@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(kFT)
     // the next launch may set up early; wait for the launch before (nothing in an ordinary launch)
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    if (gate && *gate == 0) return;
     const int tid = threadIdx.x;
     const int s = blockIdx.y / nchunks, chunk = (int)outside_in(blockIdx.y % nchunks, nchunks);
     const unsigned tile = outside_in(blockIdx.x, gridDim.x);

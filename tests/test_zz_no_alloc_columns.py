@@ -37,7 +37,7 @@ def test_many_columns_match_allocating_entry_point(cuda):
     from h3d import _lib as L
     from h3d import ops
 
-    n, h, P, npml = (64, 64, 3), (25.0, 20.0, 22.0), 9000, (6, 5, 4, 7, 1, 0)
+    n, h, P, npml = (64, 64, 3), (25.0, 20.0, 22.0), 9000, (6, 5, 4, 7, 1, 1)
     N = int(np.prod(n))
     gen = torch.Generator(device=cuda).manual_seed(4)
     wn = (2 * np.pi * 4.0) ** 2 / (1500 + 2000 * torch.rand(N, dtype=torch.float64, device=cuda, generator=gen)) ** 2
