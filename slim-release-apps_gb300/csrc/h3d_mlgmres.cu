@@ -29,8 +29,8 @@
 // the least-squares residual norm of FGMRES.m:111-113 without a host round trip; the solution y
 // is back-substituted once per cycle.  Every kernel after the matvec reads
 // a flag of the state block (the step runs / the cycle runs) and returns at once when it is
-// clear, so the host enqueues unpreconditioned cycles without waiting: it synchronises once per
-// cycle of a coarse solve there, after every fourth cycle of a smoother, and before each step of
+// clear, the matvecs of the unpreconditioned instances too, so the host enqueues unpreconditioned cycles without waiting: it synchronises once per
+// cycle of a coarse solve there, after every fourth cycle of a smoother (every one with a loose tolerance), and before each step of
 // a preconditioned instance (to decide whether the expensive preconditioner runs at all).  Sums are deterministic: fixed
 // per-thread and per-warp sums in the field's precision, then per-CTA partials and their
 // totals in FP64 in a fixed order.
@@ -1000,8 +1000,12 @@ struct Cycle {
                 smooth[i].n = n[i];
                 smooth[i].m = k[1];
                 smooth[i].nparts = parts_for(n[i]);
-                // a smoother seldom meets its tolerance: the stream is not drained after each cycle
-                smooth[i].ahead = 4;
+                // A tight tolerance is seldom met: the stream is not drained after each cycle (ms per solve,
+                // read every cycle -> every fourth, tolerance 1e-6: mixed 41 x 41 x 35 7.4 -> 7.0, 121 x 101 x
+                // 81 26.0 -> 25.3; 0.1: 8.3 -> 8.2, 25.4 -> 25.3).  A loose one is, and the launches of the
+                // cycles that are left, though they return at once, cost more than the wait (0.3: 8.3 -> 8.7,
+                // 25.6 -> 26.6; 0.5: 8.4 -> 10.4, 26.1 -> 30.2).
+                smooth[i].ahead = stol < 0.2 ? 4 : 1;
             }
             if (i >= 1) {
                 coarse[i].n = n[i];

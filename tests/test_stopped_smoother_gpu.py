@@ -32,9 +32,9 @@ def _solve_seconds(levels, R, P, b, precision, k, smooth_tol):
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_stopped_smoother_runs_no_matvecs(cuda, precision):
-    """smooth_tol = 1: the smoothers stop before their first step (FGMRES.m:88, hst = 1).  Three cycles of 16
-    steps then enqueue about 100 gated matvecs per V-cycle for the other setting's four, on 3.3 million points
-    (0.7 ms each in complex128, 40 us in complex64) beside a few milliseconds of outer and coarse work: the
+    """smooth_tol = 1: the smoothers stop before their first step (FGMRES.m:88, hst = 1).  Up to three
+    cycles of 16 steps are then enqueued for one of one step: 100 matvecs more per V-cycle, on 3.3 million points
+    (0.7 ms each in complex128, 40 us in complex64) beside a few milliseconds of outer and coarse work.  The
     solve takes three times as long or more where they run, a third longer where they return at once."""
     import torch
     from h3d import _lib as L
