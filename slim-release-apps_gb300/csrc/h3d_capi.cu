@@ -34,9 +34,10 @@ static int kacz_sweep_t(const Op<T> &op, cplx<T> *x, const cplx<T> *b, int nrhs,
         }
         (void)cudaGetLastError();  // out of memory is not sticky: fall back to the tile kernel
     }
-    // LEX on stored coefficients where they fit: a plane of rows then takes a warp's short chain per
-    // row instead of a thread's 600 FP64 instructions.  Otherwise the kernel that forms them per row.
-    if (order == H3D_ORDER_LEX) {
+    // LEX on stored coefficients where they take at most half of the free memory: a plane of rows then takes
+    // a warp's short chain per row instead of a thread's 600 FP64 instructions.  Otherwise the kernel that
+    // forms them per row.
+    if (order == H3D_ORDER_LEX && lex_coefs_fit<T>(op.N)) {
         DevBuf cb, rb;
         if (cb.alloc(sizeof(cplx<T>) * 27 * (size_t)op.N, st) == H3D_OK &&
             rb.alloc(sizeof(T) * (size_t)op.N, st) == H3D_OK) {

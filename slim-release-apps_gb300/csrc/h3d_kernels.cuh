@@ -52,6 +52,9 @@ int launch_sweep(const Op<T> &op, cplx<T> *x, const cplx<T> *b, int nrhs, T w, b
 // store_lex_coefs: t = (dx+1) + 3(dy+1) + 9(dz+1) and 1/||a_i||^2.  sweep_lex_stored: dirs gives the
 // direction t of each coefficient column (null: in order); scale holds 1/||a_i||^2 (inverse) or
 // ||a_i||^2 (null: formed from the row); couplings that leave the grid are skipped.
+// lex_coefs_fit: whether the coefficients of N rows take at most half of the free device memory.
+template <typename T>
+bool lex_coefs_fit(long long N);
 template <typename T>
 int store_lex_coefs(const Op<T> &op, bool adj, cplx<T> *coef, T *rinv, cudaStream_t st);
 template <typename T>

@@ -17,7 +17,7 @@
 // Measured on 61^3, complex128, one right-hand side with b: 41.7 -> 4.6 ms per double sweep (1562
 // planes at 2.7 us each: launch rate and the latency of x through L2 bound it now; 0.4 ms of it
 // forms the coefficients), against the kernel that forms each row in one thread (h3d_stencil.cu),
-// which stays for grids whose 27 N coefficients do not fit.
+// which stays for grids whose 27 N coefficients would take more than half of the free memory.
 #include "h3d_internal.cuh"
 #include "h3d_kernels.cuh"
 
@@ -163,6 +163,17 @@ int lex_passes(int nx, int ny, int nz, const cplx<T> *coef, const LexOffsets &of
 }  // namespace
 
 template <typename T>
+bool lex_coefs_fit(long long N)
+{
+    size_t fr = 0, tot = 0;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return sizeof(cplx<T>) * 27 * (size_t)N <= fr / 2;
+}
+
+template <typename T>
 int store_lex_coefs(const Op<T> &op, bool adj, cplx<T> *coef, T *rinv, cudaStream_t st)
 {
     const long long blocks = (op.N + kStoreT - 1) / kStoreT;
@@ -191,6 +202,8 @@ int sweep_lex_stored(int nx, int ny, int nz, const cplx<T> *coef, const unsigned
     return lex_passes<T, false>(nx, ny, nz, coef, offs, scale, x, b, nrhs, w, active, st);
 }
 
+template bool lex_coefs_fit<double>(long long);
+template bool lex_coefs_fit<float>(long long);
 template int store_lex_coefs<double>(const Op<double> &, bool, cplx<double> *, double *, cudaStream_t);
 template int store_lex_coefs<float>(const Op<float> &, bool, cplx<float> *, float *, cudaStream_t);
 template int sweep_lex_stored<double>(int, int, int, const cplx<double> *, const unsigned char[27], const double *, bool,

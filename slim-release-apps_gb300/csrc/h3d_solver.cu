@@ -188,10 +188,8 @@ struct CgRun {
         if ((rc = parts.alloc(sizeof(double) * 2 * (size_t)s.G * nrhs, st))) return rc;
         s.part = parts.as<double>();
         if (b8) return H3D_OK;  // the batch holds its own coefficients and row norms
-        if (order == H3D_ORDER_LEX) {  // stored coefficients when they take at most half of the free memory
-            size_t fr = 0, tot = 0;
-            const size_t bytes = sizeof(cplx<T>) * 27 * (size_t)N;
-            if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && bytes <= fr / 2 && coefs.alloc(bytes, st) == H3D_OK &&
+        if (order == H3D_ORDER_LEX) {
+            if (lex_coefs_fit<T>(N) && coefs.alloc(sizeof(cplx<T>) * 27 * (size_t)N, st) == H3D_OK &&
                 norms.alloc(sizeof(T) * (size_t)N, st) == H3D_OK) {
                 coef = coefs.as<cplx<T>>();
                 rinv = norms.as<T>();
