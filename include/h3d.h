@@ -218,12 +218,13 @@ int h3d_residual_noalloc(const h3d_grid *g, const double *wn_re, const double *w
 
 /* ---- diagnostics ------------------------------------------------------------------------ */
 /* Checks the bounded waits of the complex128 BLOCK8 sweep kernel on this GPU (no counterpart in the
- * reference).  Runs one double sweep on an internal 24^3 complex128 problem in which the kernel's first
- * colour step announces a coefficient copy on its mbarrier but never issues it, with every
- * wait limited to limit_ms (0 < limit_ms <= 1000): each CTA gives up after the limit, records
- * the expired wait in the sweep's status word and returns.  Returns H3D_ERR_TIMEOUT when that
- * status came back (the expected result; the context stays usable), H3D_OK if no wait
- * expired, or another status if the call itself failed.  Synchronous. */
+ * reference).  Runs two double sweeps on an internal 24^3 complex128 problem with every wait limited to
+ * limit_ms (0 < limit_ms <= 1000).  In the first, the kernel's first colour step announces a
+ * coefficient copy on its mbarrier but never issues it; in the second, which runs as one launch, the block at
+ * the origin does not publish that it is done.  The CTAs that wait give up after the limit, record the
+ * expired wait in the sweep's status word and return.  Returns H3D_ERR_TIMEOUT when that status came back
+ * from both (the expected result; the context stays usable), H3D_OK if either saw no wait expire (the error
+ * text holds both), or another status if the call itself failed.  Synchronous. */
 int h3d_check_wait_timeout(double limit_ms);
 
 /* ---- MATLAB-layout host entry points (what the drop-in MEX gateway calls) ----------- */

@@ -64,6 +64,7 @@ struct B8Batch {
     int *err = nullptr;                       // device status: H3D_ERR_TIMEOUT after an expired wait
     unsigned long long wait_limit_ns = 1000000000ull;
     int verbose = 0;
+    bool force_one_launch = false;            // complex128, whatever the number of blocks (set before configure())
 
     void add(const Op<T> &op, bool adj, long long col0, int c0, int nrhs) { items.push_back({op, adj, col0, c0, nrhs}); }
     // Any problem with a complex wavenumber.

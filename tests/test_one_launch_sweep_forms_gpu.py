@@ -1,6 +1,6 @@
 """The complex128 BLOCK8 sweep in one launch, in each of its compiled forms (right-hand sides per CTA and per
 thread, by H3D_BLOCK8_CONFIG), on grids whose blocks miss neighbours, with as many columns as take a parity
-past the GPU's SMs and the last group half filled.
+past the GPU's SMs and the last group half filled; and its wait for the blocks around, made to run out.
 
 Tolerance: the order of dependent updates is the oracle's; 54 updates of a point by 27-term FP64 sums differ
 by some 1e-14 of the field's size.
@@ -67,3 +67,15 @@ def test_one_column_matches_oracle(cuda, mode):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert sms < _blocks(n) <= 4 * sms
     _sweep_matches_oracle(cuda, n, 15, 1, mode, False)
+
+
+def test_wait_for_the_blocks_around_expires_with_a_status(cuda):
+    """Both bounded waits give up after 3 ms (the whole sweep's blocks take less than one), and a sweep right
+    after, in one launch, matches the oracle."""
+    from h3d import _lib as L
+
+    lib = L.load()
+    assert lib.h3d_check_wait_timeout(3.0) == L.ERR_TIMEOUT
+    status = str(L.ERR_TIMEOUT).encode()
+    assert b"blocks around in one launch (status " + status + b")" in lib.h3d_last_error()
+    _sweep_matches_oracle(cuda, (61, 58, 50), 5, 14, 1, False)
