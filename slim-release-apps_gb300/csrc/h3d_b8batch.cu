@@ -649,10 +649,15 @@ int B8Batch<T>::configure(int c, cudaStream_t st)
     int rc;
     desc.release();
     starts.release();
-    if ((rc = desc.alloc(sizeof(B8Prob<T>) * np, st)) || (rc = starts.alloc(sizeof(int) * hs.size(), st))) return rc;
-    // pageable sources: staged before the calls return
-    H3D_CUDA_TRY(cudaMemcpyAsync(desc.p, h.data(), sizeof(B8Prob<T>) * np, cudaMemcpyHostToDevice, st));
-    H3D_CUDA_TRY(cudaMemcpyAsync(starts.p, hs.data(), sizeof(int) * hs.size(), cudaMemcpyHostToDevice, st));
+    // A single complex64 problem's descriptor goes with each launch and it needs no tables.  (Nor copies of
+    // h and hs, which a stream capture would record to be read at each replay, when they are gone; in
+    // complex128 the call's status read refuses a capture.)
+    if (sizeof(T) == 8 || np > 1) {
+        if ((rc = desc.alloc(sizeof(B8Prob<T>) * np, st)) || (rc = starts.alloc(sizeof(int) * hs.size(), st))) return rc;
+        // pageable sources: staged before the calls return
+        H3D_CUDA_TRY(cudaMemcpyAsync(desc.p, h.data(), sizeof(B8Prob<T>) * np, cudaMemcpyHostToDevice, st));
+        H3D_CUDA_TRY(cudaMemcpyAsync(starts.p, hs.data(), sizeof(int) * hs.size(), cudaMemcpyHostToDevice, st));
+    }
     first = h[0];
     cfg = c;
     nflow = counters;
