@@ -1,7 +1,8 @@
 """The complex64 BLOCK8 sweep (one warp per z slab, windows in registers) where it can go wrong:
 block remainders of 1, 2 and 11 points on every axis, a single block, PML everywhere and nowhere
 inside a block, one, two and three right-hand sides (a full and a half-filled group), both modes,
-real and complex wavenumbers, and problems of several kinds in one batch.
+real and complex wavenumbers, and how far a NaN spreads.  (Problems of several kinds in one batch are in
+test_solver_gpu.py.)
 
 Tolerance: a row projection in complex64 has a relative error of a few FP32 roundings (6e-8 each,
 27-term sums); a point is updated by at most 27 rows per pass and two passes, so errors stay
@@ -61,3 +62,22 @@ def test_slab_sweep_keeps_nan_and_inactive_columns(cuda):
     b[1, X.shape[0] // 2] = 1.0
     u, info = solver.solve((n, h, npml), torch.as_tensor(wn.astype(np.float64), device=cuda), b, precision="mixed")
     assert bool((u[0] == 0).all()) and info["rel_res_true"] <= 1e-6
+
+
+@pytest.mark.parametrize("n,npml,at", [((300, 13, 14), 4, (0, 0, 0)), ((14, 290, 13), 5, (7, 150, 6)),
+                                       ((11, 12, 280), 3, (10, 11, 279)), ((130, 140, 13), 6, (60, 70, 12))])
+@pytest.mark.parametrize("mode,wnc", [(1, False), (2, False), (1, True)])
+def test_nan_spreads_as_far_as_in_the_oracle(cuda, n, npml, at, mode, wnc):
+    """One NaN in x, on a face, in the interior or in a corner of a grid that is long enough for the sweep not
+    to carry it everywhere: the same points turn NaN as in the sequential sweep, no others."""
+    import torch
+    from h3d import ops
+
+    h, g, wn, X, _ = _problem(n, npml, 7, wnc, 1)
+    X[at[0] + n[0] * (at[1] + n[1] * at[2]), 0] = np.nan
+    ref = O.sweep(g, wn.astype(np.complex128 if wnc else np.float64), 1.5, X, None, adj=(mode == 2),
+                  order=O.ORDER_BLOCK8, blk=(12, 12, 12), nthreads=2)
+    t = lambda a: torch.as_tensor(np.ascontiguousarray(a), device=cuda)
+    y = ops.kacz_sweep((n, h, npml), t(wn), 1.5, t(X.T), None, mode, order=3).cpu().numpy().T
+    assert 0 < np.isnan(ref).sum() < ref.size
+    np.testing.assert_array_equal(np.isnan(y), np.isnan(ref))
