@@ -25,6 +25,7 @@
 //    it still has in flight, and returns without writing its box back.  The host reads the
 //    status word and fails the call; the context stays usable.
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -484,13 +485,16 @@ int launch_b8(const B8Prob<T> *probs, const int *starts, int nprob, long long nc
 {
     constexpr size_t smem = b8_smem<T, R, S>();
     static_assert(smem + sizeof(B8Prob<T>) + 16 <= 232448, "batched BLOCK8 configuration exceeds shared memory");
-    static bool attr_set = false;  // per instantiation and process
-    if (!attr_set) {
+    static std::atomic<unsigned long long> attr_set{0};  // bit per device
+    int dev = 0;
+    H3D_CUDA_TRY(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (dev > 63 || !(attr_set.load() & bit)) {
         H3D_CUDA_TRY(cudaFuncSetAttribute(sweep_b8_kernel<T, R, RPT, S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
         H3D_CUDA_TRY(cudaFuncSetAttribute(sweep_b8_kernel<T, R, RPT, S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-        attr_set = true;
+        attr_set.fetch_or(bit);
     }
     auto *kern = flow ? sweep_b8_kernel<T, R, RPT, S, true> : sweep_b8_kernel<T, R, RPT, S, false>;
     kern<<<(unsigned)nctas, 2 * kNR * R / RPT, smem, st>>>(probs, starts, nprob, x, b, w, active, par, backward, nsteps, err,
