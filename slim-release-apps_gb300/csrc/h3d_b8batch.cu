@@ -524,7 +524,7 @@ int launch_b8_cfg(int cfg, bool wnc, const B8Prob<T> &one, const B8Prob<T> *prob
     return H3D_ERR_BAD_ARG;
 }
 
-// Tuner cache: batch shape (grid sizes, columns, precision) -> configuration.
+// Tuner cache: device and batch shape (grid sizes, columns, precision, mode, kind of wavenumber) -> configuration.
 std::mutex g_b8_mutex;
 std::map<std::vector<long long>, int> g_b8_cache;
 
@@ -751,13 +751,16 @@ template <typename T>
 int B8Batch<T>::tune(cplx<T> *y, long long len, cudaStream_t st)
 {
     const bool fp64 = sizeof(T) == 8;
-    std::vector<long long> key{(long long)sizeof(T)};
+    int dev = 0;
+    H3D_CUDA_TRY(cudaGetDevice(&dev));
+    std::vector<long long> key{dev, (long long)sizeof(T)};
     for (const Item &it : items) {
         key.push_back(it.op.nx);
         key.push_back(it.op.ny);
         key.push_back(it.op.nz);
         key.push_back(it.nrhs);
         key.push_back(it.adj);
+        key.push_back(it.op.wni != nullptr);
     }
     {
         std::lock_guard<std::mutex> lk(g_b8_mutex);
