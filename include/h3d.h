@@ -180,13 +180,14 @@ int h3d_mvp(const h3d_grid *g, const void *wn_re, const void *wn_im, const void 
 
 /* One forward + backward Kaczmarz sweep with relaxation w on x (in place), right-hand
  * side b (NULL = 0).  Same element types as h3d_mvp.  block: BLOCK / BLOCK8 block size
- * (NULL or 0 = default).  COLOUR27 and BLOCK8 with 12x12x12 blocks run on stored row
- * coefficients (about 27 N complex values of temporary device memory) whenever they fit;
+ * (NULL or 0 = default).  COLOUR27 and, in complex128, BLOCK8 with 12x12x12 blocks run on stored row
+ * coefficients (about 27 N complex values of temporary device memory) whenever they fit, BLOCK8 in
+ * complex64 on records of 18 KB a block (30 KB with a complex wavenumber);
  * block[0] == -1 selects the kernels that form the coefficients themselves (COLOUR27: the
  * shared-memory tile kernel; BLOCK8: 12x12x12 blocks).  LEX stores its coefficients (27 N + N / 2
  * complex values) where they take at most half of the free device memory.  BLOCK8 on stored coefficients reads
  * the kernel's status word back (H3D_ERR_TIMEOUT if a bounded wait expired), so that call
- * synchronises the stream; it runs the largest right-hand-side group the columns fill, or the
+ * synchronises the stream; BLOCK8 runs the largest right-hand-side group the columns fill, or the
  * configuration whose index the environment variable H3D_BLOCK8_CONFIG holds. */
 int h3d_kacz_sweep(const h3d_grid *g, const void *wn_re, const void *wn_im, double w, void *x,
                    const void *b, int nrhs, int mode, int order, const int32_t *block, int dtype,

@@ -1,13 +1,14 @@
 // Batched BLOCK8 Kaczmarz double sweep over a table of problems (h3d_b8batch.cu; the complex64
 // kernel in h3d_b8slab.cu).
 //
-// One launch per block parity (complex128: or one in all, see h3d_b8batch.cu) covers every (problem, block, group of R right-hand sides) of
-// the batch: problems may differ in grid size, PML, wavenumber (frequency) and mode, and each
-// keeps its own stored row coefficients.  A CTA finds its problem by a binary search over the
-// per-parity prefix counts of CTAs, copies the problem's descriptor into shared memory, and
-// runs the block's 27 colours (54 for the middle parity) on its shared-memory boxes, the
-// coefficient slab and inverse row norms of each colour arriving by one thread's bulk copy
-// into an S-deep ring of buffers that complete on mbarriers.
+// One launch per block parity (complex128: or one in all, see h3d_b8batch.cu) covers every (problem,
+// block, group of R right-hand sides) of the batch: problems may differ in grid size, PML, wavenumber
+// (frequency) and mode.  A CTA finds its problem by a binary search over the per-parity prefix counts of
+// CTAs, copies the problem's descriptor into shared memory, and runs the block's 27 colours (54 for the
+// middle parity) on its shared-memory boxes.  complex128: each problem keeps its stored row coefficients,
+// and the coefficient slab and inverse row norms of each colour arrive by one thread's bulk copy into an
+// S-deep ring of buffers that complete on mbarriers.  complex64: a block's record holds its inverse row
+// norms and wavenumber box, copied once; the coefficients are formed.
 #pragma once
 
 #include <memory>

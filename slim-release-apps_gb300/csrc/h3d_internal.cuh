@@ -62,7 +62,8 @@ __host__ __device__ __forceinline__ void cmac_cb(cplx<T> &acc, cplx<T> a, cplx<T
 // exactly like the scalar operation, and take a scalar register or constant as a
 // broadcast operand.  A complex value times a real scalar is then one instruction.  The
 // packed forms pay off in issue-bound kernels (the matvec); the latency-bound Kaczmarz
-// sweeps measured slower with them and keep the scalar forms.  PK selects the packed form
+// sweeps measured slower with them and keep the scalar forms (the BLOCK8 sweep of h3d_b8slab.cu, the same
+// with either, is packed).  PK selects the packed form
 // (complex64 on sm_100+ only; complex128 is always scalar).
 #if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
 #define H3D_F32X2 1

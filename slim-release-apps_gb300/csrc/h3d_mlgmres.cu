@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kThr) fg_sub_kernel(const cplx<T> *__restrict_
 
 // Step j of the cycle (0-based): H(1:j+1, j+1) = h, H(j+2, j+1) = ||w||; Givens rotations
 // replace the least-squares solve of FGMRES.m:111 (same solution and residual norm; y itself
-// is back-substituted once per cycle, by fg_xupd_kernel).  With H(j+2, j+1) = ||w|| real the
+// is back-substituted once per cycle, by back_substitute).  With H(j+2, j+1) = ||w|| real the
 // new rotation needs only reciprocal square roots (FP64 divisions and square roots are long
 // dependent sequences on this GPU): c = |a| / r, s = (a / |a|) ||w|| / r, r = sqrt(|a|^2 +
 // ||w||^2), and the quasi-residual |g(j+2)| = |s| |g(j+1)| follows without a square root.
@@ -389,7 +389,7 @@ __device__ void givens_step(FgState *st, const double *part, int nparts, int j, 
     double d = 0.0, cs = 0.0, sr = 0.0, si = 0.0, gp = 0.0, go = 0.0, gres = 0.0, rnormr0 = 0.0;
     int nhst = 0, it = 0;
     if (threadIdx.x < 32) {
-        if (row <= j) d = __ldcg(reinterpret_cast<const double *>(st->h) + threadIdx.x);  // CTA 0 of this launch wrote it
+        if (row <= j) d = __ldcg(reinterpret_cast<const double *>(st->h) + threadIdx.x);  // written by the orthogonalisation's CTA 0, maybe in this launch
         if (row < j) {
             cs = st->cs[row];
             sr = st->sn[row].re;

@@ -2,7 +2,7 @@
 //
 // A CTA owns a 32 x 4 (complex128: 32 x 8) column of rows and marches a chunk of planes in z.  Each plane of
 // x (and, forward, of the wavenumber) is staged in shared memory with its one-point xy
-// halo by asynchronous copies (double-buffered: plane p+1 streams in while plane p is
+// halo by asynchronous copies (three buffers: planes p+1 and p+2 stream in while plane p is
 // used).  From a plane every thread forms the partial sums of its 3 x 3 in-plane
 // neighbourhood that the stencil needs -- centre, the two x-faces, the two y-faces and
 // the corner pairs grouped by the sign of dx and of dy -- and keeps the last three planes

@@ -20,7 +20,7 @@
 // operations per grid point: 60 (interior), 86 (z PML), 88-144 (x or y PML), against 80, 106 and 186
 // with nine brackets per pending row, and no lanes on points outside the grid: a 61^3 grid on 32 x 8
 // column tiles ran half of its lanes there.  100 operations per point on 201 x 201 x 101 (198 before),
-// 80% of the unit's peak.  us per launch, forward, one column, against the column tiles: 17^3 36 -> 21,
+// 71% of the unit's peak over the launch.  us per launch, forward, one column, against the column tiles: 17^3 36 -> 21,
 // 31^3 61 -> 27, 61^3 186 -> 83, 101 x 101 x 51 308 -> 172, 161 x 161 x 81 842 -> 505, 201 x 201 x 101
 // 1374 -> 915.
 #pragma once

@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "h3d_b8.cuh"
+#include "h3d_b8slab.cuh"
 #include "h3d_internal.cuh"
 #include "h3d_kernels.cuh"
 #include "h3d_krylov.cuh"
@@ -571,12 +572,12 @@ static bool use_batched_block8(const std::vector<SolveProb> &P, const h3d_solve_
     const int32_t *bk = o.block;
     if (!(bk[0] <= 0 || (bk[0] == 12 && bk[1] == 12 && bk[2] == 12))) return false;
     size_t need = 0;
-    const size_t cs = o.precision == H3D_PREC_FP64 ? 16 : 8;
     for (const SolveProb &p : P) {
-        const size_t nb = (size_t)((p.g.n[0] + 11) / 12) * ((p.g.n[1] + 11) / 12) * ((p.g.n[2] + 11) / 12) * 27 * 64;
-        // complex128: stored coefficients and row norms; complex64: block records (at most 7440 floats)
-        if (o.precision == H3D_PREC_FP64) need += nb * (27 * cs + cs / 2) + (size_t)p.g.n[0] * p.g.n[1] * p.g.n[2] * (cs / 2);
-        else need += nb / (27 * 64) * 7440 * sizeof(float);
+        const int NI = (p.g.n[0] + 11) / 12, NJ = (p.g.n[1] + 11) / 12, NK = (p.g.n[2] + 11) / 12;
+        const size_t rows = (size_t)NI * NJ * NK * 27 * 64;
+        // complex128: stored coefficients and row norms; complex64: block records (the larger kind)
+        if (o.precision == H3D_PREC_FP64) need += rows * (27 * 16 + 8) + (size_t)p.g.n[0] * p.g.n[1] * p.g.n[2] * 8;
+        else need += slab_record_bytes(NI, NJ, NK, true);
     }
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
